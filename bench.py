@@ -74,19 +74,13 @@ WORKLOADS = {
                "Frobenius norm 1e-3, CRSS uniform in [tau0, 2 tau0], elastic-predictor start"),
 }
 METRIC, DESC = WORKLOADS[WORKLOAD]
-# DRAM bytes (read + write) per FP64 colour launch at 64^3, measured with ncu
-# on two launches of the profiling case and scaled per row to the mean colour
-SOR_TRAFFIC_PER_LAUNCH = 81.1e6
-# the same for the FP32-matrix colour kernel (profiles/k_sor_colour_tma_fp32_cube64.md)
-SOR32_TRAFFIC_PER_LAUNCH = 47.3e6
 CPU_STEPS = 2          # steps of the full-size checker run (cpu_baseline and oracle_error)
 INC_WARM, INC_TIMED = 5, 10   # increments leg: untimed increments, then timed ones
 POINTS = 1 << 20
 # the tuned form: FP32-matrix sweeps with FP64 residual refinement
-# (abi.FAS_MODE_SOR_FP32).  The persistent tile solve and the consistent
-# tangent are measured beside it (rooflines.sor_*tiles,
-# increments.plain_consistent_tangent) and left out: neither is faster, and
-# the tangent moves per-point stresses by up to toler's reach.
+# (abi.FAS_MODE_SOR_FP32).  The consistent tangent is measured beside it
+# (increments.plain_consistent_tangent) and left out: it is not faster, and
+# moves per-point stresses by up to toler's reach.
 TUNED_MODE = 1
 POINTS_CPU = 1 << 15   # points of the checker's bounded sample in the point workload
 
@@ -616,23 +610,19 @@ def run_gpu(args):
 def rooflines(g, start, prob) -> dict:
     """Achieved rates of the dominant kernels against the measured peaks.
 
-    * SOR colour kernels (FP64 and the tuned FP32 copy): algorithmic bytes of
-      one whole FACSLS solve -- the first step's -- over its device time with
-      the CUDA graph and programmatic launches the steps use (per-launch
-      event pairs would serialise the overlapped launches).  `launch_ms` is
-      that time per colour launch, so launches x launch_ms is the solve.
+    * SOR solve (FP64 rows, the tuned form's FP32 rows, symmetric FP32 rows):
+      algorithmic bytes of one whole FACSLS solve -- the first step's -- over
+      its device time.  `launch_ms` is that time per colour phase, so
+      launches x launch_ms is the solve.
     * k_elem (constitutive pass): the algorithmic FP64 operations counted per
       GP (fas_flops.h) over its per-launch event time, against measured DGEMM.
     """
     from cpfem_code_b200 import abi
     pk = peaks()
     out = {}
-    kernels = {"sor": "k_sor_colour_tma<double,27,4>", "sor_fp32": "k_sor_colour_tma<float,27,4>",
-               "sor_tiles": "k_sor_tiles<double>", "sor_fp32_tiles": "k_sor_tiles<float>",
+    kernels = {"sor": "k_sor_flow<double,27>", "sor_fp32": "k_sor_flow<float,27>",
                "sor_fp32_sym": "k_sor_colour_tma<float,15,8,true>"}
     for tag, mode in (("sor", abi.FAS_MODE_PLAIN), ("sor_fp32", abi.FAS_MODE_SOR_FP32),
-                      ("sor_tiles", abi.FAS_MODE_SOR_TILES),
-                      ("sor_fp32_tiles", abi.FAS_MODE_SOR_FP32 | abi.FAS_MODE_SOR_TILES),
                       ("sor_fp32_sym", abi.FAS_MODE_SOR_FP32 | abi.FAS_MODE_SOR_SYM)):
         g.upload(start)
         g.set_mode(mode)
@@ -648,13 +638,11 @@ def rooflines(g, start, prob) -> dict:
         out[tag] = {"kernel": kernels[tag],
                     "bound": "hbm", "achieved": ach, "peak": pk["hbm_gbs"], "unit": "GB/s",
                     "frac": ach / pk["hbm_gbs"], "peak_source": pk["source"],
-                    "traffic": (SOR_TRAFFIC_PER_LAUNCH if tag == "sor" else
-                                SOR32_TRAFFIC_PER_LAUNCH if tag == "sor_fp32" else None)
-                    if WORKLOAD == "cube64" else None,
+                    "traffic": None,
                     "bytes_per_launch": p["sor_bytes"] / nl, "launch_ms": p["ms_total"] / nl,
                     "launches": nl, "sweeps": int(p["sor_sweeps"]),
-                    "timed": "one FACSLS solve of Newton iteration 1 of increment 1 (CUDA graph, programmatic "
-                             "launches, stopping tests included) under one event pair"}
+                    "timed": "one FACSLS solve of Newton iteration 1 of increment 1 (packing of the rows and "
+                             "stopping tests included) under one event pair"}
     g.set_mode(abi.FAS_MODE_PLAIN)
     # the constitutive pass of a plastic Newton iteration: step 3 from the start
     from cpfem_code_b200 import NewtonStepper
@@ -902,8 +890,8 @@ def run_case(args) -> int:
       independent FCC points (4 increments, checkpoints every 2);
     * ``--case points``: ``--reps`` DSTRSS passes over ``--points`` points;
     * ``--case sweeps``: microseconds per sweep of the first FACSLS of n^3
-      cubes on every solve path (one CTA, colour kernels, tiles; FP64 and
-      FP32, and FP32 on symmetric rows), one JSON line per size.
+      cubes on every solve path (FP64, FP32, and FP32 on symmetric rows), one
+      JSON line per size.
     """
     from cpfem_code_b200 import GpuSolver, ReplayHistory, generator
     if args.case == "facsls":
@@ -927,17 +915,12 @@ def run_case(args) -> int:
     elif args.case == "sweeps":
         # us per sweep of the first FACSLS of n^3 cubes on each solve path
         from cpfem_code_b200 import abi
-        paths = {"one_cta": 0, "colour": abi.FAS_MODE_SOR_GRID,
-                 "tiles": abi.FAS_MODE_SOR_GRID | abi.FAS_MODE_SOR_TILES,
-                 "tiles_fp32": abi.FAS_MODE_SOR_GRID | abi.FAS_MODE_SOR_TILES | abi.FAS_MODE_SOR_FP32,
-                 "colour_fp32": abi.FAS_MODE_SOR_GRID | abi.FAS_MODE_SOR_FP32,
-                 "colour_fp32_sym": abi.FAS_MODE_SOR_GRID | abi.FAS_MODE_SOR_FP32 | abi.FAS_MODE_SOR_SYM}
+        paths = {"fp64": abi.FAS_MODE_SOR_GRID, "fp32": abi.FAS_MODE_SOR_GRID | abi.FAS_MODE_SOR_FP32,
+                 "fp32_sym": abi.FAS_MODE_SOR_GRID | abi.FAS_MODE_SOR_FP32 | abi.FAS_MODE_SOR_SYM}
         for n in (2, 4, 8, 12, 16, 20, 24, 32, 40, 48, 64):
             p = generator.cube_config(n=n, ninc=1, grain=1, seed=n)
             row = {"n": n, "nodes": p.nnod}
             for tag, mode in paths.items():
-                if tag == "one_cta" and p.nnod > 256:   # above it mode 0 is the grid path
-                    continue
                 g = GpuSolver(p.copy(), mode=mode)
                 g.update_node()
                 g.elvals(1, 1)

@@ -13,12 +13,14 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib", "libfasgpu.so")
-SOURCES = ["fas_capi.cu"]
-DEPS = ["fas_capi.cu", "fas_kernels.cuh", "fas_sor_tiles.cuh", "fas_device_warp.cuh", "fas_adjoint.cuh", "fas_device.cuh", "fas_flops.h", "fas_rng.h"]
+SOURCES = ["fas_capi.cu", "fas_cp.cu", "fas_cpq.cu", "fas_adj.cu"]
+DEPS = SOURCES + ["fas_kernels.cuh", "fas_layout.cuh", "fas_cp.cuh", "fas_sor_flow.cuh", "fas_device_warp.cuh",
+                  "fas_adjoint.cuh", "fas_adjoint_types.cuh", "fas_device.cuh", "fas_launch.h", "fas_flops.h", "fas_rng.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 TUNED = os.path.join(HERE, "tuned.json")
 
@@ -56,18 +58,23 @@ def build(force: bool = False, verbose: bool = False, defines: dict | None = Non
         return OUT
     os.makedirs(os.path.dirname(out), exist_ok=True)
     defs = tuned_defines() if defines is None else defines
-    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
-           "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",
-           *[f"-D{k}={v}" for k, v in sorted(defs.items())],
-           "-o", out + ".tmp", *[os.path.join(SRC, s) for s in SOURCES]]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
+    flags = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
+             "--expt-relaxed-constexpr", *(["-Xptxas=-v"] if verbose else []),
+             *[f"-D{k}={v}" for k, v in sorted(defs.items())]]
+    with tempfile.TemporaryDirectory() as tmp:      # one compiler per source, then the link
+        objs = [os.path.join(tmp, s + ".o") for s in SOURCES]
+        procs = [subprocess.Popen([nvcc(), *flags, "-c", "-o", o, os.path.join(SRC, s)], stdout=subprocess.PIPE,
+                                  stderr=subprocess.STDOUT, text=True) for s, o in zip(SOURCES, objs)]
+        logs = [p.communicate()[0] for p in procs]
+        if all(p.returncode == 0 for p in procs):
+            link = subprocess.run([nvcc(), *ARCH, "-shared", "-Xcompiler", "-fPIC", "-o", out + ".tmp", *objs],
+                                  stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+            procs.append(link)
+            logs.append(link.stdout)
+    if verbose or any(p.returncode for p in procs):
+        sys.stderr.write("".join(logs))
+    if any(p.returncode for p in procs):
         raise RuntimeError("nvcc failed")
-    if verbose:
-        sys.stderr.write(res.stderr)
     os.replace(out + ".tmp", out)
     return out
 

@@ -44,6 +44,7 @@
 // segment is then swept backwards.
 #pragma once
 
+#include "fas_adjoint_types.cuh"
 #include "fas_device.cuh"
 
 namespace fasdev {
@@ -159,10 +160,6 @@ __device__ __forceinline__ void tens_rot_d(const double r[3], const Dual a[6], D
         b[i + 3] = rot[0][j] * tmp[0][k] + rot[1][j] * tmp[1][k] + rot[2][j] * tmp[2][k];
     }
 }
-
-// The ampar(k) entries the parameter adjoint covers (1-based k = 1, 2, 3, 5).
-constexpr int ADJ_NP = 4;
-__host__ __device__ constexpr int adj_ampar_index(int j) { return j < 3 ? j : 4; }
 
 // Inputs of one increment's local system, as dual numbers.
 template <int NS> struct AdjIn {
@@ -455,15 +452,6 @@ __device__ __forceinline__ double objective_seed(const double *e9, int ns, const
 }
 
 // ------------------------------------------------------------ the replay
-// The history and objective of a replay.  de: de(6, ngps, ninc), dr:
-// dr(3, ngps, ninc), dt: dt(ninc), w / y: per GP.
-struct ReplayDev {
-    const double *de, *dr, *dt, *w, *y;
-    double q[3];
-    int ninc, chk;
-    int zs;          // stride (in rows of ngps) of one state record: 9 + the widest ns
-};
-
 // One replayed increment of GP g (above): DSTRSS from st and the state in
 // G.sv, then the commit.  st becomes the new stress, G.sv the new state;
 // xg receives the signed converged slips (|g| = srate dt, the sign of

@@ -13,8 +13,8 @@
 
 #include "../../include/fasolt_gpu.h"
 #include "fas_kernels.cuh"
-#include "fas_sor_tiles.cuh"
-#include "fas_adjoint.cuh"
+#include "fas_sor_flow.cuh"
+#include "fas_launch.h"
 
 #include <algorithm>
 #include <climits>
@@ -158,13 +158,21 @@ struct fas_handle {
     DVec<int> work_order, work_hist;   // work-sorted constitutive launch order
     DVec<int> cp_queue;          // head of the constitutive pass's device queue
     DVec<int> gp_item;           // GP of item e*npg + g (quadratic elements; -1 for ties)
-    // tile layout of the persistent SOR solve (k_sor_tiles; 27-slot rows)
-    int ntiles = 0;
-    DVec<int> tseg, tadj_ptr, tadj, tsrc, tbcol, tprog;
-    DVec<double> tblk64, trdiag, tpart, sol_scr;
-    DVec<float> tblk32;
-    DVec<TileSync> tsync;
-    int tile_keep_rows = 0;      // rows per tile whose blocks stay in L2 across sweeps
+    // tile layout of the persistent SOR solve (k_sor_flow), set up with the
+    // block layout; values, index words and extras on the first solve of a
+    // value type
+    int fl_nt = 0;               // 0: no tile layout, the colour kernels serve this mesh
+    bool fl_ok64 = false, fl_ok32 = false;   // the tiles fit shared memory in FP64 / FP32
+    DVec<int> fl_trow, fl_seg, fl_hptr, fl_hseg, fl_hrow, fl_src, fl_node, fl_tile;
+    DVec<uint16_t> fl_lcol, fl_head;
+    DVec<unsigned char> fl_from;
+    bool fl_early = false;       // late columns are kept apart (FlowRow)
+    DVec<unsigned> fl_voff64, fl_voff32, fl_eoff;
+    DVec<int> fl_cptr64, fl_cptr32;
+    size_t fl_nrec64 = 0, fl_nrec32 = 0;      // their bytes
+    DVec<unsigned char> fl_rec64, fl_rec32;   // the chunks' records
+    DVec<double> fl_old;
+    DVec<ulonglong2> fl_sync;    // published values, then the tiles' shares
     // NRITER of an increment as one CUDA graph (FAS_MODE_GRAPH): loop state,
     // report lines, the instantiated graph of each increment, and the two
     // side streams its nested loop bodies are captured on
@@ -177,7 +185,7 @@ struct fas_handle {
     cudaGraphExec_t sor_graph = nullptr;   // GRAPH_SWEEPS plain sweeps
     cudaGraphExec_t sor32_graph = nullptr; // one refinement cycle of the FP32 form
     bool sor32_graph_sym = false;          // ... on the symmetric rows
-    bool blk32_fresh = false;    // the last assembly wrote blk32
+    bool fp32_fresh = false;     // the last assembly ran in FAS_MODE_SOR_FP32
     // reductions and control
     std::vector<int> sor_boff, sor_nblk;       // FP64 colour grids and their partial offsets
     std::vector<int> sor_boff32, sor_nblk32;   // FP32 colour grids (smaller rings, more CTAs)
@@ -365,8 +373,8 @@ int greedy_colouring(fas_handle *h, const std::vector<double> &xyz)
     return 0;
 }
 
-int build_tiles(fas_handle *h, const std::vector<double> &xyz, const std::vector<int> &bcol_host,
-                const std::vector<int> &nslot_host, const std::vector<int> &rowof_host);
+int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<int> &bcol_host,
+               const std::vector<int> &nslot_host, const std::vector<int> &rowof_host);
 
 // Row permutation by colour, node block neighbourhoods and the per-slot
 // element-local index words; allocates the block matrix.
@@ -513,119 +521,245 @@ int build_layout(fas_handle *h, const std::vector<double> &xyz)
     CK(h->d_cstart.put(h->col_start.data(), h->ncol + 1, s));
     h->sor_small = nn <= (h->slots == SLOTS ? SOR_SMALL_ROWS : SOR_SMALL_ROWS81);
     CK(cudaStreamSynchronize(s));
-    return build_tiles(h, xyz, bcol, nslot, rowof);
+    return build_flow(h, xyz, bcol, nslot, rowof);
 }
 
-// Recursive coordinate bisection of nodes[lo, hi) into nt tiles t0 ..
-// t0 + nt - 1 of (nearly) equal node counts: cut across the longest extent
-// of the bounding box, in proportion to the tiles on each side.
-void rcb_tiles(std::vector<int> &nodes, int lo, int hi, int t0, int nt, const std::vector<double> &xyz,
-               std::vector<int> &tile_of)
+// Recursive coordinate bisection into nt tiles t0 .. t0 + nt - 1: cut across
+// the longest extent of the bounding box, in proportion to the tiles on each
+// side.  Every colour's nodes (nodes[lo[c], hi[c])) are cut in that proportion
+// by themselves, so that each tile has its share of every colour: a phase of
+// the solve handles one colour and is as long as its largest share.  `carry`
+// keeps the colours' rounding from adding up.
+void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::vector<int> &hi, int t0, int nt,
+               const std::vector<double> &xyz, bool by_colour, std::vector<int> &tile_of)
 {
-    if (nt <= 1 || hi - lo <= 1) {
-        for (int k = lo; k < hi; ++k) tile_of[nodes[k]] = t0;
+    const int nc = (int)lo.size();
+    if (nt <= 1) {
+        for (int c = 0; c < nc; ++c)
+            for (int k = lo[c]; k < hi[c]; ++k) tile_of[nodes[k]] = t0;
         return;
     }
     double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    for (int k = lo; k < hi; ++k)
-        for (int c = 0; c < 3; ++c) {
-            mn[c] = std::min(mn[c], xyz[3 * (size_t)nodes[k] + c]);
-            mx[c] = std::max(mx[c], xyz[3 * (size_t)nodes[k] + c]);
-        }
+    for (int c = 0; c < nc; ++c)
+        for (int k = lo[c]; k < hi[c]; ++k)
+            for (int d = 0; d < 3; ++d) {
+                mn[d] = std::min(mn[d], xyz[3 * (size_t)nodes[k] + d]);
+                mx[d] = std::max(mx[d], xyz[3 * (size_t)nodes[k] + d]);
+            }
     int ax = 0;
-    for (int c = 1; c < 3; ++c)
-        if (mx[c] - mn[c] > mx[ax] - mn[ax]) ax = c;
+    for (int d = 1; d < 3; ++d)
+        if (mx[d] - mn[d] > mx[ax] - mn[ax]) ax = d;
     const int ntl = nt / 2;
-    const int cut = lo + (int)((long long)(hi - lo) * ntl / nt);
-    std::nth_element(nodes.begin() + lo, nodes.begin() + cut, nodes.begin() + hi, [&](int a, int b) {
+    std::vector<int> cut(nc);
+    auto before = [&](int a, int b) {
         const double xa = xyz[3 * (size_t)a + ax], xb = xyz[3 * (size_t)b + ax];
         return xa != xb ? xa < xb : a < b;
-    });
-    rcb_tiles(nodes, lo, cut, t0, ntl, xyz, tile_of);
-    rcb_tiles(nodes, cut, hi, t0 + ntl, nt - ntl, xyz, tile_of);
+    };
+    if (!by_colour) {
+        std::vector<int> all;
+        for (int c = 0; c < nc; ++c) all.insert(all.end(), nodes.begin() + lo[c], nodes.begin() + hi[c]);
+        const size_t at = all.size() * (size_t)ntl / nt;
+        if (at < all.size()) {
+            std::nth_element(all.begin(), all.begin() + at, all.end(), before);
+            const int pivot = all[at];
+            for (int c = 0; c < nc; ++c)
+                cut[c] = (int)(std::partition(nodes.begin() + lo[c], nodes.begin() + hi[c],
+                                              [&](int m) { return before(m, pivot); }) -
+                               nodes.begin());
+        } else
+            cut = hi;
+    }
+    long long carry = 0;
+    for (int c = 0; c < nc && by_colour; ++c) {
+        const long long want = (long long)(hi[c] - lo[c]) * ntl + carry;
+        const long long take = std::min<long long>(std::max<long long>((want + nt / 2) / nt, 0), hi[c] - lo[c]);
+        carry = want - take * nt;
+        cut[c] = lo[c] + (int)take;
+        if (cut[c] > lo[c] && cut[c] < hi[c])
+            std::nth_element(nodes.begin() + lo[c], nodes.begin() + cut[c], nodes.begin() + hi[c], before);
+    }
+    rcb_tiles(nodes, lo, cut, t0, ntl, xyz, by_colour, tile_of);
+    rcb_tiles(nodes, cut, hi, t0 + ntl, nt - ntl, xyz, by_colour, tile_of);
 }
 
-// Tile layout of the persistent SOR solve (k_sor_tiles): one spatial tile
-// of nodes per SM, rows ordered tile by tile and colour by colour inside a
-// tile, the column ids marked by colour order, and the tiles each tile
-// depends on.  27-slot rows only; other layouts keep the colour kernels.
-int build_tiles(fas_handle *h, const std::vector<double> &xyz, const std::vector<int> &bcol_host,
-                const std::vector<int> &nslot_host, const std::vector<int> &rowof_host)
+// Tile layout of the persistent SOR solve (k_sor_flow): one spatial tile of
+// nodes per CTA, its rows by colour (rows that other tiles read first), the
+// tile-local index of every column, and the halo: the nodes of other tiles
+// that the tile's rows read, by colour.  A mesh with more colours than the
+// kernel's tables, or tiles whose solution values leave no room for a copy
+// ring (about 90^3 8-node bricks per GPU in FP64), keeps the colour kernels.
+template <typename T, int S> bool flow_fits(int n, int nh)
 {
-    if (h->slots != SLOTS || h->ncol > TILE_MAXCOL) return 0;
-    const int nn = h->nnod, ncol = h->ncol, crow = crow_of(SLOTS);
-    int occ = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sor_tiles<double>, 32 * tile_warps<double>(),
-                                                     tile_smem_bytes<double>()));
-    int occ32 = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ32, k_sor_tiles<float>, 32 * tile_warps<float>(),
-                                                     tile_smem_bytes<float>()));
-    if (occ < 1 || occ32 < 1) return 0;   // the colour kernels serve this device
-    const int nt = std::min(h->nsm, std::max(1, nn / 64));
-    std::vector<int> nodes(nn), tile_of(nn, 0);
-    for (int i = 0; i < nn; ++i) nodes[i] = i;
-    rcb_tiles(nodes, 0, nn, 0, nt, xyz, tile_of);
-    // rows: tile, then colour, then node id
-    std::vector<int> order(nn);
-    for (int i = 0; i < nn; ++i) order[i] = i;
-    std::sort(order.begin(), order.end(), [&](int a, int b) {
-        if (tile_of[a] != tile_of[b]) return tile_of[a] < tile_of[b];
-        if (h->h_colour[a] != h->h_colour[b]) return h->h_colour[a] < h->h_colour[b];
-        return a < b;
-    });
-    std::vector<int> tseg((size_t)nt * (ncol + 1), 0), tsrc(nn), tbcol((size_t)crow * nn, 0);
+    using L = FlowRow<T, S>;
+    size_t o = L::F32 ? (size_t)n * 24 + (size_t)(n + nh) * 12 : (size_t)(n + nh) * 24;
+    o += (size_t)nh * 4 + (S == SLOTS ? 0 : (size_t)((n + L::CH - 1) / L::CH + 1) * 4);
+    o = (o + 127) & ~(size_t)127;
+    return n + nh < 65536 && o + 3 * (size_t)L::SLOT <= (size_t)FLOW_SMEM;
+}
+
+// f(slots) with the slots as a compile-time constant
+template <typename F> auto flow_shape(int slots, F &&f)
+{
+    return slots == SLOTS ? f(std::integral_constant<int, SLOTS>{}) : f(std::integral_constant<int, SLOTS20>{});
+}
+
+// Bytes of FP64 rows up to which the solve runs as one tile: one SM then
+// needs no exchange with others, and its phases (a CTA barrier each) stay
+// shorter than the 0.5 us an exchange takes.
+constexpr long long FLOW_ONE_TILE_BYTES = 700 * 1024;
+// Rows per tile up to which every colour is cut evenly by itself: phases of a
+// few rows are as long as their largest share (us per sweep evenly against
+// by position: 32^3 18.4 against 19.7, 21 x 17 x 23 20-node bricks 46.9
+// against 50.8), while the larger halo of the ragged cuts costs a large tile a
+// slot of its ring (64^3 95.5 against 88.9, 32^3 20-node 163 against 149).
+constexpr long long FLOW_EVEN_ROWS = 512;
+// Rows per tile below which a mesh gets fewer tiles than SMs.
+constexpr int FLOW_MIN_ROWS = 16;
+
+int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<int> &bcol_host,
+               const std::vector<int> &nslot_host, const std::vector<int> &rowof_host)
+{
+    if (h->ncol > FLOW_MAXCOL) return 0;
+    const int nn = h->nnod, ncol = h->ncol, S = h->slots, crow = crow_of(S);
+    const int nt = (long long)nn * brow_of(S) * 8 <= FLOW_ONE_TILE_BYTES
+                       ? 1
+                       : std::min(h->nsm, std::max(1, nn / FLOW_MIN_ROWS));
+    std::vector<int> nodes(nn), tile_of(nn, 0), clo(h->col_start.begin(), h->col_start.end() - 1),
+        chi(h->col_start.begin() + 1, h->col_start.end());
+    for (int m = 0; m < nn; ++m) nodes[rowof_host[m]] = m;   // by colour
+    rcb_tiles(nodes, clo, chi, 0, nt, xyz, nn < FLOW_EVEN_ROWS * nt, tile_of);
+    std::vector<unsigned char> shared(nn, 0);   // the node is read by another tile
+    for (int m = 0; m < nn; ++m) {
+        const int *c = &bcol_host[(size_t)rowof_host[m] * crow];
+        const int ns = nslot_host[rowof_host[m]];
+        for (int sl = 1; sl < ns && !shared[m]; ++sl) shared[m] = tile_of[c[sl]] != tile_of[m];
+    }
+    // rows: tile, colour, shared first, node id (a counting sort on the
+    // first three, stable in the node id)
+    const size_t nkey = (size_t)nt * ncol * 2;
+    auto key = [&](int m) { return ((size_t)tile_of[m] * ncol + h->h_colour[m]) * 2 + (shared[m] ? 0 : 1); };
+    std::vector<int> first(nkey + 1, 0), order(nn), rowt(nn), trow(nt + 1), seg((size_t)nt * (ncol + 1));
+    for (int m = 0; m < nn; ++m) ++first[key(m) + 1];
+    for (size_t k = 0; k < nkey; ++k) first[k + 1] += first[k];
+    for (int t = 0; t <= nt; ++t) trow[t] = first[(size_t)t * ncol * 2];
+    for (int t = 0; t < nt; ++t)
+        for (int c = 0; c <= ncol; ++c) seg[(size_t)t * (ncol + 1) + c] = first[((size_t)t * ncol + c) * 2] - trow[t];
     {
-        std::vector<int> cnt((size_t)nt * ncol, 0);
-        for (int n = 0; n < nn; ++n) ++cnt[(size_t)tile_of[n] * ncol + h->h_colour[n]];
-        int r = 0;
-        for (int t = 0; t < nt; ++t) {
-            for (int c = 0; c < ncol; ++c) {
-                tseg[(size_t)t * (ncol + 1) + c] = r;
-                r += cnt[(size_t)t * ncol + c];
-            }
-            tseg[(size_t)t * (ncol + 1) + ncol] = r;
+        std::vector<int> at(first.begin(), first.end() - 1);
+        for (int m = 0; m < nn; ++m) {
+            rowt[m] = at[key(m)]++;
+            order[rowt[m]] = m;
         }
     }
-    std::vector<std::vector<int>> adj(nt);
-    for (int r = 0; r < nn; ++r) {
-        const int n = order[r], p = rowof_host[n], t = tile_of[n];
-        tsrc[r] = p;
-        const int ns = nslot_host[p];
-        for (int sl = 0; sl < ns; ++sl) {
-            const int m = bcol_host[(size_t)p * crow + sl];
-            unsigned w = (unsigned)m;
-            if (h->h_colour[m] < h->h_colour[n]) w |= TILE_LOWER;
-            tbcol[(size_t)r * crow + sl] = (int)w;
-            if (tile_of[m] != t) adj[t].push_back(tile_of[m]);
-        }
-        tbcol[(size_t)r * crow + SLOTS] = ns;
+    // halo of every tile by colour, and the tile-local columns
+    std::vector<int> hptr(nt + 1, 0), hseg((size_t)nt * (ncol + 1), 0), hrow, src(nn), tile(nn), stamp(nn, -1), hidx(nn, 0);
+    std::vector<uint16_t> lcol((size_t)nn * S, 0), head(nn);
+    std::vector<unsigned char> from((size_t)nn * S, 0xFF);
+    std::vector<int> halo;
+    // whether late columns are kept apart (FlowRow): not in a mesh where some row
+    // has more of them than the format holds
+    bool early = true;
+    const int most = S == SLOTS ? FlowRow<double, SLOTS>::LATE : FlowRow<double, SLOTS20>::LATE;
+    for (int m = 0; m < nn && early; ++m) {
+        const int p = rowof_host[m], before = (h->h_colour[m] + ncol - 1) % ncol;
+        int nl = 0;
+        for (int sl = 1; sl < nslot_host[p]; ++sl) nl += h->h_colour[bcol_host[(size_t)p * crow + sl]] == before;
+        early = nl <= most;
     }
-    std::vector<int> aptr(nt + 1, 0), alist;
+    bool ok64 = true, ok32 = true;
     for (int t = 0; t < nt; ++t) {
-        std::sort(adj[t].begin(), adj[t].end());
-        adj[t].erase(std::unique(adj[t].begin(), adj[t].end()), adj[t].end());
-        if ((int)adj[t].size() > TILE_MAXADJ) return 0;   // the colour kernels serve this mesh
-        aptr[t + 1] = aptr[t] + (int)adj[t].size();
-        alist.insert(alist.end(), adj[t].begin(), adj[t].end());
+        const int n = trow[t + 1] - trow[t];
+        halo.clear();
+        for (int r = trow[t]; r < trow[t + 1]; ++r) {
+            const int m = order[r], p = rowof_host[m];
+            src[r] = p;
+            tile[r] = t;
+            const int *c = &bcol_host[(size_t)p * crow];
+            for (int sl = 1; sl < nslot_host[p]; ++sl)
+                if (tile_of[c[sl]] != t && stamp[c[sl]] != t) {
+                    stamp[c[sl]] = t;
+                    halo.push_back(c[sl]);
+                }
+        }
+        std::sort(halo.begin(), halo.end(), [&](int a, int b) {
+            return h->h_colour[a] != h->h_colour[b] ? h->h_colour[a] < h->h_colour[b] : rowt[a] < rowt[b];
+        });
+        const int nh = (int)halo.size();
+        hptr[t + 1] = hptr[t] + nh;
+        for (int k = 0, c = 0; c <= ncol; ++c) {
+            while (k < nh && h->h_colour[halo[k]] < c) ++k;
+            hseg[(size_t)t * (ncol + 1) + c] = c == ncol ? nh : k;
+        }
+        for (int k = 0; k < nh; ++k) {
+            hidx[halo[k]] = n + k;
+            hrow.push_back(rowt[halo[k]]);
+        }
+        ok64 = ok64 && flow_shape(S, [&](auto s) { return flow_fits<double, s()>(n, nh); });
+        ok32 = ok32 && flow_shape(S, [&](auto s) { return flow_fits<float, s()>(n, nh); });
+        if (!ok64 && !ok32) return 0;
+        for (int r = trow[t]; r < trow[t + 1]; ++r) {
+            const int p = src[r], ns = nslot_host[p];
+            const int *c = &bcol_host[(size_t)p * crow];
+            const int before = (h->h_colour[order[r]] + ncol - 1) % ncol;
+            auto is_late = [&](int sl) { return early && sl > 0 && h->h_colour[c[sl]] == before; };
+            int nl = 0, e = 0, l = 0;
+            for (int sl = 0; sl < ns; ++sl) nl += is_late(sl);
+            head[r] = (uint16_t)((ns - nl) | (nl << 7) | (shared[order[r]] ? 0x8000 : 0));
+            for (int sl = 0; sl < ns; ++sl) {
+                const int pos = is_late(sl) ? S - 1 - l++ : e++;
+                const int at = S == SLOTS ? FlowRow<double, SLOTS>::stored(pos, ns - nl, nl)
+                                          : FlowRow<double, SLOTS20>::stored(pos, ns - nl, nl);
+                from[(size_t)r * S + at] = (unsigned char)sl;
+                lcol[(size_t)r * S + at] = (uint16_t)(tile_of[c[sl]] == t ? rowt[c[sl]] - trow[t] : hidx[c[sl]]);
+            }
+        }
     }
+    // value offsets of 81-slot rows, packed to their own slot counts
+    std::vector<unsigned> vo64(nn + 1, 0), vo32(nn + 1, 0);
+    for (int r = 0; r < nn; ++r) {
+        const unsigned nv = 9u * (unsigned)nslot_host[src[r]];
+        vo64[r + 1] = vo64[r] + (nv * 8 + 15) / 16;
+        vo32[r + 1] = vo32[r] + (nv * 4 + 15) / 16;
+    }
+    // first chunk of every tile, and the records' bytes
+    std::vector<int> cp64(nt + 1, 0), cp32(nt + 1, 0);
+    flow_shape(S, [&](auto sl) {
+        using L64 = FlowRow<double, sl()>;
+        using L32 = FlowRow<float, sl()>;
+        for (int t = 0; t < nt; ++t) {
+            cp64[t + 1] = cp64[t] + (trow[t + 1] - trow[t] + L64::CH - 1) / L64::CH;
+            cp32[t + 1] = cp32[t] + (trow[t + 1] - trow[t] + L32::CH - 1) / L32::CH;
+        }
+        h->fl_nrec64 = (size_t)cp64[nt] * (S == SLOTS ? L64::SLOT : L64::HB) + (S == SLOTS ? 0 : (size_t)vo64[nn] * 16);
+        h->fl_nrec32 = (size_t)cp32[nt] * (S == SLOTS ? L32::SLOT : L32::HB) + (S == SLOTS ? 0 : (size_t)vo32[nn] * 16);
+    });
     cudaStream_t s = h->stream;
-    h->ntiles = nt;
-    CKA(h->tseg.alloc(tseg.size()));
-    CKA(h->tadj_ptr.alloc(aptr.size()));
-    CKA(h->tadj.alloc(std::max<size_t>(alist.size(), 1)));
-    CKA(h->tsrc.alloc(nn));
-    CKA(h->tbcol.alloc(tbcol.size()));
-    CKA(h->tprog.alloc(nt));
-    CKA(h->tpart.alloc((size_t)TILE_SLOTS_SYNC * nt * 2));
-    CKA(h->tsync.alloc(1));
-    CKA(h->trdiag.alloc((size_t)3 * nn));
-    CKA(h->sol_scr.alloc((size_t)3 * nn));
-    CK(h->tseg.put(tseg.data(), tseg.size(), s));
-    CK(h->tadj_ptr.put(aptr.data(), aptr.size(), s));
-    if (!alist.empty()) CK(h->tadj.put(alist.data(), alist.size(), s));
-    CK(h->tsrc.put(tsrc.data(), nn, s));
-    CK(h->tbcol.put(tbcol.data(), tbcol.size(), s));
+    auto up = [&](auto &dst, const auto &v) -> int {
+        CKA(dst.alloc(std::max<size_t>(v.size(), 1)));
+        CK(dst.put(v.data(), v.size(), s));
+        return 0;
+    };
+    int rc = up(h->fl_trow, trow);
+    if (!rc) rc = up(h->fl_seg, seg);
+    if (!rc) rc = up(h->fl_hptr, hptr);
+    if (!rc) rc = up(h->fl_hseg, hseg);
+    if (!rc) rc = up(h->fl_hrow, hrow);
+    if (!rc) rc = up(h->fl_src, src);
+    if (!rc) rc = up(h->fl_node, order);
+    if (!rc) rc = up(h->fl_cptr64, cp64);
+    if (!rc) rc = up(h->fl_cptr32, cp32);
+    if (!rc) rc = up(h->fl_tile, tile);
+    if (!rc) rc = up(h->fl_lcol, lcol);
+    if (!rc) rc = up(h->fl_head, head);
+    if (!rc) rc = up(h->fl_from, from);
+    if (!rc && S != SLOTS) rc = up(h->fl_voff64, vo64);
+    if (!rc && S != SLOTS) rc = up(h->fl_voff32, vo32);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(s));
+    h->fl_nt = nt;
+    h->fl_early = early;
+    h->fl_ok64 = ok64;
+    h->fl_ok32 = ok32;
     return 0;
 }
 
@@ -763,10 +897,14 @@ int create_impl(fas_handle *h, const fas_mesh_desc *Md, const fas_matl_desc *T, 
                             cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem_bytes<float, SLOTS20>()));
     CK(cudaFuncSetAttribute(k_sor_colour_tma<float, SLOTS_SYM, TMA_LPR_SYM, true>,
                             cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem_bytes<float, SLOTS_SYM>()));
-    CK(cudaFuncSetAttribute(k_sor_tiles<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            tile_smem_bytes<double>()));
-    CK(cudaFuncSetAttribute(k_sor_tiles<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            tile_smem_bytes<float>()));
+    for (int slots : {SLOTS, SLOTS20})
+        CK(flow_shape(slots, [](auto sl) {
+            const cudaError_t e =
+                cudaFuncSetAttribute(k_sor_flow<double, sl()>, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
+            return e != cudaSuccess
+                       ? e
+                       : cudaFuncSetAttribute(k_sor_flow<float, sl()>, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
+        }));
     CK(cudaMallocHost((void **)&h->hc, sizeof(HostCtl)));
     CK(cudaEventCreate(&h->ev_t0));
     CK(cudaEventCreate(&h->ev_t1));
@@ -1067,6 +1205,8 @@ int down_field(fas_handle *h, void *dst, int rb, int ld, int nk, int n, const do
     return 0;
 }
 
+int prepare_solve(fas_handle *h);
+
 int upload_impl(fas_handle *h, const fas_state_desc *S)
 {
     if (!S || (S->real_bytes != 4 && S->real_bytes != 8)) return FAS_E_ARG;
@@ -1106,6 +1246,7 @@ int upload_impl(fas_handle *h, const fas_state_desc *S)
         std::vector<double> xyz(nd3);
         for (int i = 0; i < nd3; ++i) xyz[i] = rdv(S->x, rb, i);
         rc = build_layout(h, xyz);
+        if (!rc) rc = prepare_solve(h);
         if (rc) return rc;
     }
     CK(cudaStreamSynchronize(h->stream));
@@ -1199,36 +1340,29 @@ template <typename K> unsigned cp_grid(fas_handle *h, K kern, long long n, int *
     return std::min<unsigned>(full, (unsigned)occ * (unsigned)h->nsm);
 }
 
-template <int NS> int launch_elem(fas_handle *h, int inc, int nit)
+int launch_elem(fas_handle *h, int inc, int nit)
 {
     Span sp(h, &h->P.ms_constitutive);
+    const int ns = h->ns_tmpl;
+    const double dt = h->h_tiem[inc - 1];
+    int *queue = nullptr, bs = 128;
     if (h->nn != 8) {   // quadratic elements: one thread per (element, GP)
-        auto go = [&](auto kern) {
-            const long long nit_items = (long long)h->npg * h->nlmnt;
-            const int *order = work_order(h, (int)nit_items, h->gp_item.p);
-            int *queue = nullptr, bs = 128;
-            const unsigned grid = cp_grid(h, kern, nit_items, &queue, &bs);
-            kern<<<grid, bs, h->stage_bytes, h->stream>>>(h->mesh(), h->M, h->C, h->gp(), h->dnq.p, h->wfac, h->x.p, h->dx.p,
-                                              h->rec.p, h->h_tiem[inc - 1], inc, nit, h->ekey.p, order, queue);
-        };
-        if (h->nn == 20)
-            go(k_elemq<NS, 20, 8>);
-        else if (h->nn == 10)
-            go(k_elemq<NS, 10, 4>);
-        else
-            go(k_elemq<NS, 15, 6>);
-    }
-    else if (!(h->mode & FAS_MODE_CP_WARP)) {
+        const auto kern = elemq_kernel(ns, h->nn);
+        const long long items = (long long)h->npg * h->nlmnt;
+        const int *order = work_order(h, (int)items, h->gp_item.p);
+        const unsigned grid = cp_grid(h, kern, items, &queue, &bs);
+        kern<<<grid, bs, h->stage_bytes, h->stream>>>(h->mesh(), h->M, h->C, h->gp(), h->dnq.p, h->wfac, h->x.p,
+                                                      h->dx.p, h->rec.p, dt, inc, nit, h->ekey.p, order, queue);
+    } else if ((h->mode & FAS_MODE_CP_WARP) && ns <= 32) {   // more than 32 systems: one thread per GP only
+        elem_wc_kernel(ns)<<<nblocks(32LL * h->nlmnt, 128), 128, 0, h->stream>>>(
+            h->mesh(), h->M, h->C, h->gp(), h->x.p, h->dx.p, h->rec.p, dt, inc, nit, h->ekey.p);
+    } else {
+        const auto kern = elem_kernel(ns);
         const int *order = work_order(h, h->nlmnt, h->gpe.p);
-        int *queue = nullptr, bs = 128;
-        const unsigned grid = cp_grid(h, k_elem<NS>, h->nlmnt, &queue, &bs);
-        k_elem<NS><<<grid, bs, h->stage_bytes, h->stream>>>(
-            h->mesh(), h->M, h->C, h->gp(), h->x.p, h->dx.p, h->rec.p, h->h_tiem[inc - 1], inc, nit, h->ekey.p,
-            order, queue);
+        const unsigned grid = cp_grid(h, kern, h->nlmnt, &queue, &bs);
+        kern<<<grid, bs, h->stage_bytes, h->stream>>>(h->mesh(), h->M, h->C, h->gp(), h->x.p, h->dx.p, h->rec.p, dt,
+                                                      inc, nit, h->ekey.p, order, queue);
     }
-    else
-        k_elem_wc<(NS > 12 ? 32 : 12)><<<nblocks(32LL * h->nlmnt, 128), 128, 0, h->stream>>>(
-            h->mesh(), h->M, h->C, h->gp(), h->x.p, h->dx.p, h->rec.p, h->h_tiem[inc - 1], inc, nit, h->ekey.p);
     sp.end();
     keep(h, sp);
     LAUNCHED(h);
@@ -1241,13 +1375,18 @@ template <int NS> int launch_elem(fas_handle *h, int inc, int nit)
 // Returns the first element's FAFERR code in element order, if any.
 int ensure_fp32(fas_handle *h)
 {
-    if (!(h->mode & FAS_MODE_SOR_FP32) || h->blk32.p || h->point_mode) return 0;
+    if (!(h->mode & FAS_MODE_SOR_FP32) || h->point_mode) return 0;
     const size_t nd3 = 3 * (size_t)h->nnod;
-    CKA(h->blk32.alloc((size_t)brow_of(h->slots) * h->nnod));
-    CKA(h->sor_d.alloc(nd3));
-    CKA(h->sor_d32.alloc(nd3));
-    CKA(h->sor_r.alloc(nd3));
-    CK(h->blk32.zero(h->stream));
+    if (!h->sor_d.p) {
+        CKA(h->sor_d.alloc(nd3));
+        CKA(h->sor_r.alloc(nd3));
+    }
+    if (!h->sor_d32.p && (!h->fl_ok32 || (h->mode & FAS_MODE_SOR_SYM))) CKA(h->sor_d32.alloc(nd3));
+    // the colour kernels' FP32 rows; the persistent kernel packs its own
+    if (!h->blk32.p && !h->fl_ok32) {
+        CKA(h->blk32.alloc((size_t)brow_of(h->slots) * h->nnod));
+        CK(h->blk32.zero(h->stream));
+    }
     return 0;
 }
 
@@ -1319,18 +1458,7 @@ int elvals_impl(fas_handle *h, int inc, int nit, bool bc)
     if (int rc = ensure_sym(h)) return rc;
     CK(cudaMemsetAsync(h->ekey.p, 0xFF, sizeof(unsigned long long), s));
     CK(cudaMemsetAsync(h->flags.p, 0, sizeof(int), s));
-    int rc;
-    switch (h->ns_tmpl) {
-    case 12: rc = launch_elem<12>(h, inc, nit); break;
-    case 32: rc = launch_elem<32>(h, inc, nit); break;
-    default: {   // more than 32 systems: one thread per GP only
-        const uint32_t m = h->mode;
-        h->mode &= ~FAS_MODE_CP_WARP;
-        rc = launch_elem<60>(h, inc, nit);
-        h->mode = m;
-    } break;
-    }
-    if (rc) return rc;
+    if (const int rc = launch_elem(h, inc, nit)) return rc;
     {
         Span sp(h, &h->P.ms_assembly);
         const long long nthr = (long long)h->slots * h->nnod;   // thread (row, slot), row-major
@@ -1347,7 +1475,7 @@ int elvals_impl(fas_handle *h, int inc, int nit, bool bc)
         keep(h, sp);
         LAUNCHED(h);
         h->P.n_assembly++;
-        h->blk32_fresh = h->block().blk32 != nullptr;
+        h->fp32_fresh = (h->mode & FAS_MODE_SOR_FP32) && h->sor_d.p;
         h->P.assembly_bytes += h->asm_bytes;
     }
     CK(cudaMemcpyAsync(h->hc->ekey, h->ekey.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -1487,12 +1615,10 @@ void launch_fold(fas_handle *h)
                                                                       h->sor_acc.p, (int)nacc);
 }
 
-// Start of an FP32 solve: whether its sweeps take the symmetric rows, and
-// if so their packing from the assembled FP64 rows and zero accumulators
-// (the correction starts at zero).
+// Start of an FP32 solve on symmetric rows: their packing from the assembled
+// FP64 rows and zero accumulators (the correction starts at zero).
 void sym_begin(fas_handle *h, const BlockDev &B)
 {
-    h->sym_on = h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM) && (h->mode & FAS_MODE_SOR_FP32);
     if (!h->sym_on) return;
     k_sym_pack<<<nblocks(32LL * h->nnod, 256), 256, 0, h->stream>>>(B, h->sym_mask.p, h->blk_sym.p, h->bcol_sym.p);
     cudaMemsetAsync(h->sor_acc.p, 0, (size_t)4 * h->nnod * sizeof(float), h->stream);
@@ -1554,104 +1680,160 @@ int ensure_fp32_graph(fas_handle *h, const BlockDev &B, double tolerl)
     return 0;
 }
 
-// One cooperative launch of the persistent tile solve: at most maxsw
-// sweeps from sol0, sweep counts reported from sweep_base on.
-template <typename T>
-int launch_tiles(fas_handle *h, const T *blk, const double *rhs, const double *base, const double *rdiag,
-                 double *sol0, int maxsw, int sweep_base, double tolerl)
+// ---------------------------------------------------------------- persistent solve
+// Whether the FP64 / FP32 solve runs as the persistent tile kernel.
+bool flow_on(const fas_handle *h, bool fp32)
 {
-    cudaStream_t s = h->stream;
-    CK(h->tprog.zero(s));
-    CK(h->tsync.zero(s));
-    TileArgs<T> a;
-    a.blk = blk;
-    a.bcol = h->tbcol.p;
-    a.tseg = h->tseg.p;
-    a.tadj_ptr = h->tadj_ptr.p;
-    a.tadj = h->tadj.p;
-    a.rhs = rhs;
-    a.base = base;
-    a.rdiag = rdiag;
-    a.sol0 = sol0;
-    a.sol1 = h->sol_scr.p;
-    a.progress = h->tprog.p;
-    a.part = h->tpart.p;
-    a.sync = h->tsync.p;
+    return h->fl_nt > 0 && (fp32 ? h->fl_ok32 && !h->sym_on : h->fl_ok64);
+}
+
+template <typename T> struct FlowBufs;
+template <> struct FlowBufs<double> {
+    static DVec<unsigned char> &rec(fas_handle *h) { return h->fl_rec64; }
+    static size_t bytes(fas_handle *h) { return h->fl_nrec64; }
+    static unsigned *voff(fas_handle *h) { return h->fl_voff64.p; }
+    static int *cptr(fas_handle *h) { return h->fl_cptr64.p; }
+};
+template <> struct FlowBufs<float> {
+    static DVec<unsigned char> &rec(fas_handle *h) { return h->fl_rec32; }
+    static size_t bytes(fas_handle *h) { return h->fl_nrec32; }
+    static unsigned *voff(fas_handle *h) { return h->fl_voff32.p; }
+    static int *cptr(fas_handle *h) { return h->fl_cptr32.p; }
+};
+
+// Buffers of the persistent solve in value type T, sized on its first use
+// and kept (the pattern is fixed), with the rows' index words.
+template <typename T> int ensure_flow(fas_handle *h)
+{
+    using B = FlowBufs<T>;
+    const size_t R = h->nnod;
+    if (!h->fl_old.p) CKA(h->fl_old.alloc(3 * R));
+    if (!h->fl_sync.p) CKA(h->fl_sync.alloc(3 * R + 8 * (size_t)h->fl_nt));
+    if (sizeof(T) == 4 && !h->fl_eoff.p) CKA(h->fl_eoff.alloc(R));
+    if (B::rec(h).p) return 0;
+    CKA(B::rec(h).alloc(B::bytes(h)));
+    return flow_shape(h->slots, [&](auto sl) -> int {
+        k_flow_meta<T, sl()><<<nblocks((long long)R * FlowRow<T, sl()>::LPR, 256), 256, 0, h->stream>>>(
+            (int)R, h->fl_lcol.p, h->fl_head.p, h->fl_from.p, B::voff(h), h->fl_tile.p, h->fl_trow.p, B::cptr(h),
+            h->fl_node.p, B::rec(h).p, sizeof(T) == 4 ? h->fl_eoff.p : nullptr);
+        LAUNCHED(h);
+        return 0;
+    });
+}
+
+// The buffers that the solves of the handle's mode will use, with the block
+// layout: a first solve then costs what the others do (another mode's are
+// allocated on its first solve).
+int prepare_solve(fas_handle *h)
+{
+    if (int rc = ensure_fp32(h)) return rc;
+    if (h->fl_nt == 0) return 0;
+    const bool fp32 = (h->mode & FAS_MODE_SOR_FP32) && !(h->sor_small && !(h->mode & FAS_MODE_SOR_GRID));
+    if (fp32 && h->fl_ok32 && !(h->mode & FAS_MODE_SOR_SYM)) return ensure_flow<float>(h);
+    return !fp32 && h->fl_ok64 ? ensure_flow<double>(h) : 0;
+}
+
+// Start of a solve: the assembled rows packed into tile order, no value
+// published yet.
+template <typename T> int flow_begin(fas_handle *h, const BlockDev &B)
+{
+    const unsigned blk = (unsigned)std::min<long long>(nblocks(h->nnod, 8), (long long)h->nsm * 16);
+    const auto kern = flow_shape(h->slots, [](auto sl) { return &k_flow_pack<T, sl()>; });
+    kern<<<blk, 256, 0, h->stream>>>(B, h->fl_src.p, FlowBufs<T>::voff(h), h->fl_tile.p, h->fl_trow.p,
+                                     FlowBufs<T>::cptr(h), h->fl_from.p, h->rhs.p, FlowBufs<T>::rec(h).p);
+    LAUNCHED(h);
+    CK(h->fl_sync.zero(h->stream));
+    return 0;
+}
+
+// One cooperative launch: at most maxsw sweeps from zero, the result in
+// `sol`, sweeps counted on from ctl->sweeps.
+template <typename T> int launch_flow(fas_handle *h, double *sol, int maxsw, double tolerl)
+{
+    FlowArgs<T> a;
+    a.rec = FlowBufs<T>::rec(h).p;
+    a.voff = FlowBufs<T>::voff(h);
+    a.trow = h->fl_trow.p;
+    a.cptr = FlowBufs<T>::cptr(h);
+    a.seg = h->fl_seg.p;
+    a.hseg = h->fl_hseg.p;
+    a.hptr = h->fl_hptr.p;
+    a.hrow = h->fl_hrow.p;
+    a.node = h->fl_node.p;
+    a.gx = h->fl_sync.p;
+    a.part = h->fl_sync.p + 3 * (size_t)h->nnod;
+    a.old = h->fl_old.p;
+    a.sol = sol;
     a.ctl = h->sorctl.p;
-    a.ntiles = h->ntiles;
+    a.ntiles = h->fl_nt;
     a.ncol = h->ncol;
     a.maxsw = maxsw;
-    a.sweep_base = sweep_base;
+    a.early = h->fl_early ? 1 : 0;
     a.tolerl = tolerl;
-    a.keep_rows = h->tile_keep_rows;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(h->ntiles);
-    cfg.blockDim = dim3(32 * tile_warps<T>());
-    cfg.dynamicSmemBytes = tile_smem_bytes<T>();
-    cfg.stream = s;
+    cfg.gridDim = dim3(h->fl_nt);
+    cfg.blockDim = dim3(FLOW_THREADS);
+    cfg.dynamicSmemBytes = FLOW_SMEM;
+    cfg.stream = h->stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, k_sor_tiles<T>, a));
+    CK(cudaLaunchKernelEx(&cfg, flow_shape(h->slots, [](auto sl) { return &k_sor_flow<T, sl()>; }), a));
     LAUNCHED(h);
     return 0;
 }
 
-// FACSLS by the persistent tile kernel: the assembled rows are copied into
-// the tile layout, then one launch runs the FP64 solve to convergence; the
-// FP32 form runs refinement cycles of refine_every sweeps (one launch, the
-// fold and the FP64 residual each).  Leaves the verdict in h->hc->sor.
-int facsls_tiles(fas_handle *h, const BlockDev &B, double tolerl, bool fp32)
+// One refinement cycle of the FP32 form on the persistent kernel: `sweeps`
+// FP32 sweeps on the correction, the fold into the iterate, and the FP64
+// residual, which also goes into the rows' extras for the next cycle.
+int launch_flow_cycle(fas_handle *h, const BlockDev &B, double tolerl, int sweeps)
+{
+    Span sp(h, &h->P.ms_sor_colour);
+    if (int rc = launch_flow<float>(h, h->sor_d.p, sweeps, tolerl)) return rc;
+    sp.end();
+    keep(h, sp);
+    const int nd3 = 3 * h->nnod;
+    k_fold<<<nblocks(nd3, 256), 256, 0, h->stream>>>(nd3, h->ddx.p, h->sor_d.p, nullptr);
+    LAUNCHED(h);
+    const unsigned rblk = (unsigned)std::min<long long>(nblocks(h->nnod, 8), (long long)h->nsm * 8);
+    k_residual<<<rblk, 256, 0, h->stream>>>(B, h->rhs.p, h->ddx.p, h->sor_r.p, h->sorctl.p,
+                                            reinterpret_cast<double *>(h->fl_rec32.p), h->fl_eoff.p);
+    LAUNCHED(h);
+    return 0;
+}
+
+// FACSLS by the persistent kernel: one launch for the FP64 solve; cycles of
+// refine_every sweeps for the FP32 form, the host reading the flag after
+// 1, 2, 4, 4, ... cycles.  Leaves the verdict in h->hc->sor.
+int facsls_flow(fas_handle *h, const BlockDev &B, double tolerl, bool fp32)
 {
     cudaStream_t s = h->stream;
-    const int rows = h->nnod;
-    const size_t nd3 = 3 * (size_t)rows;
-    const unsigned pblk = (unsigned)std::min<long long>(nblocks(rows, 8), (long long)h->nsm * 8);
     if (!fp32) {
-        if (!h->tblk64.p) CKA(h->tblk64.alloc((size_t)BROW * rows));
-        k_tile_pack<double><<<pblk, 256, 0, s>>>(B, h->tsrc.p, rows, h->tblk64.p, h->trdiag.p);
-        LAUNCHED(h);
+        if (int rc = ensure_flow<double>(h)) return rc;
+        if (int rc = flow_begin<double>(h, B)) return rc;
         Span sp(h, &h->P.ms_sor_colour);
-        const int rc = launch_tiles<double>(h, h->tblk64.p, h->rhs.p, nullptr, FAS_SOR_RCP ? h->trdiag.p : nullptr,
-                                            h->ddx.p, 1000, 0, tolerl);
+        if (int rc = launch_flow<double>(h, h->ddx.p, 1000, tolerl)) return rc;
         sp.end();
         keep(h, sp);
-        if (rc) return rc;
         CK(cudaMemcpyAsync(&h->hc->sor, h->sorctl.p, sizeof(SorCtl), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         return 0;
     }
-    if (!h->tblk32.p) CKA(h->tblk32.alloc((size_t)BROW * rows));
-    k_tile_pack<float><<<pblk, 256, 0, s>>>(B, h->tsrc.p, rows, h->tblk32.p, nullptr);
-    LAUNCHED(h);
-    // x (= ddx) starts at 0, so the first residual is rhs itself
-    CK(cudaMemcpyAsync(h->sor_r.p, h->rhs.p, nd3 * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemsetAsync(h->sor_d.p, 0, nd3 * sizeof(double), s));
-        CK(cudaMemsetAsync(h->sor_d32.p, 0, nd3 * sizeof(float), s));
-    const int m = h->refine_every;
-    const unsigned rblk = (unsigned)std::min<long long>(nblocks(rows, 8), (long long)h->nsm * 8);
-    int done = 0, outer_per_chunk = 1;
-    while (done < 1000) {
-        for (int o = 0; o < outer_per_chunk && done < 1000; ++o) {
-            const int k = std::min(m, 1000 - done);
-            Span sp(h, &h->P.ms_sor_colour);
-            const int rc = launch_tiles<float>(h, h->tblk32.p, h->sor_r.p, h->ddx.p, nullptr, h->sor_d.p, k, done,
-                                               tolerl);
-            sp.end();
-            keep(h, sp);
-            if (rc) return rc;
-            k_fold<<<nblocks((long long)nd3, 256), 256, 0, s>>>((int)nd3, h->ddx.p, h->sor_d.p, h->sor_d32.p);
-            LAUNCHED(h);
-            k_residual<<<rblk, 256, 0, s>>>(B, h->rhs.p, h->ddx.p, h->sor_r.p, h->sorctl.p);
-            LAUNCHED(h);
+    if (int rc = ensure_flow<float>(h)) return rc;
+    if (int rc = flow_begin<float>(h, B)) return rc;
+    int per_read = 1;
+    for (int done = 0; done < 1000;) {
+        for (int o = 0; o < per_read && done < 1000; ++o) {
+            const int k = std::min(h->refine_every, 1000 - done);
+            if (int rc = launch_flow_cycle(h, B, tolerl, k)) return rc;
             done += k;
         }
         CK(cudaMemcpyAsync(&h->hc->sor, h->sorctl.p, sizeof(SorCtl), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (h->hc->sor.conv || h->hc->sor.fault) break;
-        outer_per_chunk = std::min(outer_per_chunk * 2, 4);
+        per_read = std::min(per_read * 2, 4);
     }
     return 0;
 }
@@ -1674,29 +1856,18 @@ int facsls_impl(fas_handle *h, int *sweeps, double *error)
     if (h->hc->ekey[1] != ~0ull) return 903;
     const double tolerl = h->C.toler * h->C.toler;
     const bool small = h->sor_small && !(h->mode & FAS_MODE_SOR_GRID);
-    const bool tiles = !small && h->ntiles > 0 && (h->mode & FAS_MODE_SOR_TILES);
-    if (!small && !tiles && FAS_SOR_RCP) {
+    const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->fp32_fresh;
+    h->sym_on = fp32 && h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM);
+    const bool flow = flow_on(h, fp32);
+    int done = 0, chunk = 4;
+    if (flow) {
+        if (const int rc = facsls_flow(h, B, tolerl, fp32)) return rc;
+        done = 1000;
+    } else if (FAS_SOR_RCP) {
         k_rdiag<<<nblocks(h->nnod, 256), 256, 0, s>>>(B, h->rdiag.p);
         LAUNCHED(h);
     }
-    if (small) {
-        Span sp(h, &h->P.ms_sor_colour);
-        launch_sor_small(h, B, h->sorctl.p, tolerl);
-        sp.end();
-        keep(h, sp);
-        LAUNCHED(h);
-        CK(cudaMemcpyAsync(&h->hc->sor, h->sorctl.p, sizeof(SorCtl), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-    }
-    int done = small ? 1000 : 0, chunk = 4;
-    const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->blk32.p && h->blk32_fresh;
-    if (tiles) {
-        const int rc = facsls_tiles(h, B, tolerl, fp32);
-        if (rc) return rc;
-        done = 1000;
-    }
-    h->sym_on = false;
-    if (fp32 && !tiles) {
+    if (fp32 && !flow) {
         // x (= ddx) starts at 0, so the first residual is rhs itself
         CK(cudaMemcpyAsync(h->sor_r.p, h->rhs.p, nd3 * sizeof(double), cudaMemcpyDeviceToDevice, s));
         CK(cudaMemsetAsync(h->sor_d.p, 0, nd3 * sizeof(double), s));
@@ -1768,7 +1939,7 @@ int facsls_impl(fas_handle *h, int *sweeps, double *error)
     settle_spans(h);
     const int nsw = h->hc->sor.sweeps;
     h->P.sor_sweeps += nsw;
-    h->P.n_sor_colour += small ? 1 : (int64_t)nsw * h->ncol;
+    h->P.n_sor_colour += (int64_t)nsw * h->ncol;
     double bytes = 0.0;
     for (double b : h->col_bytes) bytes += b;
     if (fp32) {   // FP32 blocks: 36 + 4 bytes per slot, plus the xs read
@@ -1890,10 +2061,17 @@ template <typename F> int capture_into(fas_handle *h, cudaStream_t &side, cudaGr
     return e == cudaSuccess ? 0 : FAS_E_CUDA;
 }
 
+// Whether the solves of a graph-launched NRITER run in the FP32 form (its
+// assemblies then run in it too).
+bool graph_fp32(const fas_handle *h)
+{
+    return (h->mode & FAS_MODE_SOR_FP32) && h->sor_d.p && !(h->sor_small && !(h->mode & FAS_MODE_SOR_GRID));
+}
+
 // One Newton iteration (nr_step_impl) with no host read: ELVALS + SUVALS,
 // FACSLS's prologue, the sweeps in a conditional node that runs only when
-// nothing failed so far (a while loop of GRAPH_SWEEPS sweeps per pass, or
-// the one-CTA solve under an if), the norms, the decision and the
+// nothing failed so far (the persistent solve under an if, its FP32 cycles
+// or GRAPH_SWEEPS sweeps of colour kernels per pass of a while loop), the norms, the decision and the
 // correction.  Issued on h->stream while it captures the body of the
 // increment graph's Newton loop `hnr`.
 int capture_nr_body(fas_handle *h, int inc, cudaGraphConditionalHandle hnr)
@@ -1903,17 +2081,7 @@ int capture_nr_body(fas_handle *h, int inc, cudaGraphConditionalHandle hnr)
     const int64_t l0 = h->launches;
     CK(cudaMemsetAsync(h->ekey.p, 0xFF, sizeof(unsigned long long), h->stream));
     CK(cudaMemsetAsync(h->flags.p, 0, sizeof(int), h->stream));
-    int rc;
-    switch (h->ns_tmpl) {
-    case 12: rc = launch_elem<12>(h, inc, 0); break;
-    case 32: rc = launch_elem<32>(h, inc, 0); break;
-    default: {
-        const uint32_t m = h->mode;
-        h->mode &= ~FAS_MODE_CP_WARP;
-        rc = launch_elem<60>(h, inc, 0);
-        h->mode = m;
-    } break;
-    }
+    int rc = launch_elem(h, inc, 0);
     if (rc) return rc;
     cudaStream_t s = h->stream;
     {
@@ -1936,17 +2104,17 @@ int capture_nr_body(fas_handle *h, int inc, cudaGraphConditionalHandle hnr)
     k_diag_check<<<nblocks(h->nnod, 256), 256, 0, s>>>(B, h->ekey.p + 1);
     LAUNCHED(h);
     const double tolerl = h->C.toler * h->C.toler;
-    const bool small = h->sor_small && !(h->mode & FAS_MODE_SOR_GRID);
-    if (!small && FAS_SOR_RCP) {
+    // the FP32 solve (facsls_impl): cycles of refine_every sweeps, each closed
+    // by the fold and the FP64 residual
+    const bool fp32 = graph_fp32(h), flow = flow_on(h, fp32);
+    const int m = h->refine_every, full = (1000 / m) * m, rest = 1000 - full;
+    if (flow) {
+        if (int r = fp32 ? flow_begin<float>(h, B) : flow_begin<double>(h, B)) return r;
+    } else if (FAS_SOR_RCP) {
         k_rdiag<<<nblocks(h->nnod, 256), 256, 0, s>>>(B, h->rdiag.p);
         LAUNCHED(h);
     }
-    // the FP32 solve (facsls_impl): cycles of refine_every sweeps on the
-    // FP32 copy, each closed by the fold and the FP64 residual
-    const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->blk32.p;
-    const int m = h->refine_every, full = (1000 / m) * m, rest = 1000 - full;
-    h->sym_on = false;
-    if (fp32) {
+    if (fp32 && !flow) {
         CK(cudaMemcpyAsync(h->sor_r.p, h->rhs.p, nd3 * sizeof(double), cudaMemcpyDeviceToDevice, s));
         CK(cudaMemsetAsync(h->sor_d.p, 0, nd3 * sizeof(double), s));
         CK(cudaMemsetAsync(h->sor_d32.p, 0, nd3 * sizeof(float), s));
@@ -1962,17 +2130,19 @@ int capture_nr_body(fas_handle *h, int inc, cudaGraphConditionalHandle hnr)
     int ncolours = 0;
     for (int c = 0; c < h->ncol; ++c) ncolours += h->col_start[c + 1] > h->col_start[c];
     cudaGraph_t sbody = nullptr;
-    if (int r = add_conditional(s, hsor, small ? cudaGraphCondTypeIf : cudaGraphCondTypeWhile, &sbody)) return r;
+    if (int r = add_conditional(s, hsor, flow && !fp32 ? cudaGraphCondTypeIf : cudaGraphCondTypeWhile, &sbody)) return r;
     rc = capture_into(h, h->cap3, sbody, [&]() -> int {
-        if (small) {
-            launch_sor_small(h, B, h->sorctl.p, tolerl);
-            LAUNCHED(h);
-            return 0;
+        if (flow && !fp32) {
+            h->g_pass_launches = 1;
+            return launch_flow<double>(h, h->ddx.p, 1000, tolerl);
         }
         if (fp32) {
-            launch_fp32_cycle(h, B, tolerl, m);
+            if (flow) {
+                if (int r = launch_flow_cycle(h, B, tolerl, m)) return r;
+            } else
+                launch_fp32_cycle(h, B, tolerl, m);
             k_sor_cycle_cond<<<1, 32, 0, h->stream>>>(h->sorctl.p, full, rest, hsor, hlast);
-            h->g_pass_launches = (int64_t)m * (ncolours + 1) + 3;
+            h->g_pass_launches = flow ? 4 : (int64_t)m * (ncolours + 1) + 3;
         } else {
             for (int it = 0; it < GRAPH_SWEEPS; ++it) {
                 for (int c = 0; c < h->ncol; ++c) launch_colour(h, c, false);
@@ -1989,6 +2159,7 @@ int capture_nr_body(fas_handle *h, int inc, cudaGraphConditionalHandle hnr)
         cudaGraph_t lbody = nullptr;
         if (int r = add_conditional(s, hlast, cudaGraphCondTypeIf, &lbody)) return r;
         rc = capture_into(h, h->cap3, lbody, [&]() -> int {
+            if (flow) return launch_flow_cycle(h, B, tolerl, rest);
             launch_fp32_cycle(h, B, tolerl, rest);
             CK(cudaGetLastError());
             return 0;
@@ -2025,7 +2196,12 @@ int ensure_inc_graph(fas_handle *h, int inc, cudaGraphExec_t *out)
     if (!h->nrrep.p) CKA(h->nrrep.alloc((size_t)std::max(h->C.maxit, 1)));
     if (!h->cp_queue.p) CKA(h->cp_queue.alloc(1));
     if (int rc = ensure_fp32(h)) return rc;
-    // the work-order buffers are sized outside the capture
+    if (int rc = ensure_sym(h)) return rc;
+    const bool fp32 = graph_fp32(h);
+    h->sym_on = fp32 && h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM);
+    // the solve's and the work order's buffers are sized outside the capture
+    if (flow_on(h, fp32))
+        if (int rc = fp32 ? ensure_flow<float>(h) : ensure_flow<double>(h)) return rc;
     if (h->nn != 8)
         work_order(h, h->npg * h->nlmnt, h->gp_item.p);
     else if (!(h->mode & FAS_MODE_CP_WARP))
@@ -2084,9 +2260,8 @@ int nriter_graph_impl(fas_handle *h, int inc, fas_iter_report *rep, int cap, int
     if (rep)
         for (int k = 0; k < std::min(n, cap); ++k) rep[k] = r[k];
     // the counters of the iterations the graph ran
-    const bool small = h->sor_small && !(h->mode & FAS_MODE_SOR_GRID);
-    const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->blk32.p;
-    const int per_pass = fp32 ? h->refine_every : GRAPH_SWEEPS;
+    const bool fp32 = graph_fp32(h), flow = flow_on(h, fp32);
+    const int per_pass = fp32 ? h->refine_every : flow ? 1000 : GRAPH_SWEEPS;
     double bytes = 0.0;
     for (double b : fp32 ? h->col_bytes32 : h->col_bytes) bytes += b;
     h->launches += 1 + (int64_t)nr.nit * h->g_body_launches;   // cumslip, and every iteration's body
@@ -2098,15 +2273,15 @@ int nriter_graph_impl(fas_handle *h, int inc, fas_iter_report *rep, int cap, int
         h->P.assembly_bytes += h->asm_bytes;
         h->P.sor_sweeps += sw;
         h->P.sor_bytes += bytes * sw;
-        h->P.n_sor_colour += small ? 1 : (int64_t)sw * h->ncol;
-        if (!small) h->launches += (int64_t)((sw + per_pass - 1) / per_pass) * h->g_pass_launches;
+        h->P.n_sor_colour += (int64_t)sw * h->ncol;
+        h->launches += (int64_t)((sw + per_pass - 1) / per_pass) * h->g_pass_launches;
     }
     return nr.status;
 }
 
 int nriter_impl(fas_handle *h, int inc, fas_iter_report *rep, int cap, int *n_rep)
 {
-    if ((h->mode & FAS_MODE_GRAPH) && !(h->mode & FAS_MODE_SOR_TILES) && h->prof < 2)
+    if ((h->mode & FAS_MODE_GRAPH) && h->prof < 2)
         return nriter_graph_impl(h, inc, rep, cap, n_rep);
     int nit = 0;
     bool l_conv = true;
@@ -2256,20 +2431,18 @@ int replay_block(const fas_handle *h)
 
 // The forward sweep; with rs > 0 it also records the last segment for
 // the reverse sweep.
-template <int NS>
 void launch_replay_fwd(fas_handle *h, const ReplayDev &H, const DevGp &G, int rs)
 {
     const int bs = replay_block(h);
-    k_replay_fwd<NS><<<nblocks(h->ngps, bs), bs, 0, h->stream>>>(h->M, h->C, G, h->gp_iel.p, h->st.p, H,
+    replay_fwd_kernel(h->ns_tmpl)<<<nblocks(h->ngps, bs), bs, 0, h->stream>>>(h->M, h->C, G, h->gp_iel.p, h->st.p, H,
                                                                   h->rp.chk.p, rs > 0 ? h->rp.rec.p : nullptr,
                                                                   rs, h->rp.jg.p, h->rp.eq.p, h->ekey.p);
 }
 
-template <int NS>
 void launch_replay_adj(fas_handle *h, const ReplayDev &H, const DevGp &G, int rs)
 {
     const int bs = replay_block(h);
-    k_replay_adj<NS><<<nblocks(h->ngps, bs), bs, 0, h->stream>>>(h->M, h->C, G, h->gp_iel.p, H, h->rp.chk.p,
+    replay_adj_kernel(h->ns_tmpl)<<<nblocks(h->ngps, bs), bs, 0, h->stream>>>(h->M, h->C, G, h->gp_iel.p, H, h->rp.chk.p,
                                                                   h->rp.rec.p, rs, h->rp.jg.p, h->rp.gst.p,
                                                                   h->rp.gsv.p, h->rp.gp.p, h->ekey.p);
 }
@@ -2491,35 +2664,16 @@ int32_t fas_gpu_constitutive(fas_handle *h, int32_t inc, int32_t nit)
     CK(cudaMemsetAsync(h->ekey.p, 0xFF, sizeof(unsigned long long), s));
     Span sp(h, &h->P.ms_constitutive);
     const double dt = h->h_tiem[inc - 1];
-    const unsigned nbw = nblocks(32LL * h->ngps, 128);
-    const bool thr = !(h->mode & FAS_MODE_CP_WARP) || h->maxns > 32;
-    const int *order = thr ? work_order(h, h->ngps, nullptr) : nullptr;
-    switch (h->ns_tmpl) {
-    case 12:
-        if (thr) {
-            int *queue = nullptr;
-            int bs = 128;
-            const unsigned grid = cp_grid(h, k_points<12>, h->ngps, &queue, &bs);
-            k_points<12><<<grid, bs, h->stage_bytes, s>>>(h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p, order, queue);
-        }
-        else k_points_wc<12><<<nbw, 128, 0, s>>>(h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p);
-        break;
-    case 32:
-        if (thr) {
-            int *queue = nullptr;
-            int bs = 128;
-            const unsigned grid = cp_grid(h, k_points<32>, h->ngps, &queue, &bs);
-            k_points<32><<<grid, bs, h->stage_bytes, s>>>(h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p, order, queue);
-        }
-        else k_points_wc<32><<<nbw, 128, 0, s>>>(h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p);
-        break;
-    default: {
-        int *queue = nullptr;
-        int bs = 128;
-        const unsigned grid = cp_grid(h, k_points<60>, h->ngps, &queue, &bs);
-        k_points<60><<<grid, bs, h->stage_bytes, s>>>(h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p, order, queue);
-        break;
-    }
+    if ((h->mode & FAS_MODE_CP_WARP) && h->maxns <= 32) {
+        points_wc_kernel(h->ns_tmpl)<<<nblocks(32LL * h->ngps, 128), 128, 0, s>>>(
+            h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p);
+    } else {
+        const auto kern = points_kernel(h->ns_tmpl);
+        const int *order = work_order(h, h->ngps, nullptr);
+        int *queue = nullptr, bs = 128;
+        const unsigned grid = cp_grid(h, kern, h->ngps, &queue, &bs);
+        kern<<<grid, bs, h->stage_bytes, s>>>(h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p,
+                                              order, queue);
     }
     sp.end();
     keep(h, sp);
@@ -2590,8 +2744,7 @@ int32_t fas_gpu_adjoint_forward(fas_handle *h, const fas_replay_desc *d, double 
     int rs = 0;
     int rc = replay_prepare(h, d, false, H, G, rs);
     if (rc) return rc;
-    if (h->ns_tmpl == 12) launch_replay_fwd<12>(h, H, G, 0);
-    else launch_replay_fwd<32>(h, H, G, 0);
+    launch_replay_fwd(h, H, G, 0);
     LAUNCHED(h);
     rc = replay_finish(h, J);
     if (rc) return rc;
@@ -2608,13 +2761,11 @@ int32_t fas_gpu_adjoint_grad(fas_handle *h, const fas_replay_desc *d, double *J,
     int rc = replay_prepare(h, d, true, H, G, rs);
     if (rc) return rc;
     const size_t ng = h->ngps;
-    if (h->ns_tmpl == 12) launch_replay_fwd<12>(h, H, G, rs);
-    else launch_replay_fwd<32>(h, H, G, rs);
+    launch_replay_fwd(h, H, G, rs);
     LAUNCHED(h);
     // the reverse sweep starts from the same twin state as the forward one
     CK(cudaMemcpyAsync(h->rp.twinsys.p, h->twinsys.p, ng * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
-    if (h->ns_tmpl == 12) launch_replay_adj<12>(h, H, G, rs);
-    else launch_replay_adj<32>(h, H, G, rs);
+    launch_replay_adj(h, H, G, rs);
     LAUNCHED(h);
     rc = replay_finish(h, J);
     if (rc) return rc;

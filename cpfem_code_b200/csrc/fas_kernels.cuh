@@ -17,9 +17,8 @@
 //     the diagonal block; bcol[row*crow + slot] is the column node and
 //     bcol[row*crow + S] the row's slot count (crow = 28 or 84).
 //
-// Kernels: the element pass (k_elem, k_elemq, the opt-in warp variants),
-// the work-sorted launch order of the constitutive kernels (k_work_*), the
-// row-gather assembly with fused SUVALS (k_assemble), the SOR colour phase
+// Kernels: the work-sorted launch order of the constitutive kernels
+// (k_work_*; the kernels themselves are in fas_cp.cuh), the row-gather assembly with fused SUVALS (k_assemble), the SOR colour phase
 // streamed by the bulk-copy engine (k_sor_colour_tma, launched with
 // programmatic serialisation) and its stopping test (k_sor_check), the
 // one-CTA solve of small meshes (k_sor_small), the FP32 refinement pieces,
@@ -28,267 +27,11 @@
 
 #include <type_traits>
 
+#include "../../include/fasolt_gpu.h"
 #include "fas_device.cuh"
-#include "fas_device_warp.cuh"
+#include "fas_layout.cuh"
 
 namespace fasdev {
-
-// Gauss-point record of an NN-node element: sfd (3 NN), stress (6),
-// weight, pad, tangent upper triangle (21), pad.
-template <int NN> struct RecLayout {
-    static constexpr int S = 3 * NN, W = 3 * NN + 6, D = 3 * NN + 8, LEN = 3 * NN + 32;
-};
-constexpr int REC = RecLayout<8>::LEN;   // 56 doubles per 8-node element record
-constexpr int REC_S = RecLayout<8>::S, REC_W = RecLayout<8>::W, REC_D = RecLayout<8>::D;
-constexpr int SLOTS = 27;        // node blocks per row of an 8-node brick mesh
-constexpr int SLOTS20 = 81;      // node blocks per row of a 20-node brick mesh
-constexpr int MAXADJ = 64;       // elements per node the tables allow (bytes of a local-index word)
-
-// block matrix addressing: a row of S slots holds 9 S values padded to a
-// multiple of 4 (so FP64 and FP32 rows are both 16-byte multiples, as bulk
-// copies need) and S column ids plus the slot count padded to a multiple of 4
-__host__ __device__ constexpr int brow_of(int S) { return (S * 9 + 3) / 4 * 4; }
-__host__ __device__ constexpr int crow_of(int S) { return (S + 1 + 3) / 4 * 4; }
-constexpr int BROW = brow_of(SLOTS);   // 244
-constexpr int CROW = crow_of(SLOTS);   // 28
-static_assert(BROW == 244 && CROW == 28, "8-node row layout");
-
-// upper-triangle index of chi(i,j), i <= j (0-based)
-__host__ __device__ __forceinline__ int utri(int i, int j) { return i * 6 - (i * (i - 1)) / 2 + (j - i); }
-
-struct MeshDev {
-    int nlmnt, nnod;
-    int nn, npg;         // nodes and Gauss points per element (8, 1 or 20, 8)
-    const int *ln;       // [nn][nlmnt] 0-based node ids
-    const int *gpe;      // [npg][nlmnt] 0-based GPs of the element
-    const int *le;       // [nlmnt]
-    const int *lt;       // [nlmnt] element type: the family's (12 or 22), or 1-6 for a tie
-    const int *ib;       // [nnod]
-    const int *ne_elem;  // [maxadj][nnod] adjacent elements, ascending
-    const int *ne_loc;   // [maxadj][nnod] local index of the node in it
-    const int *ne_cnt;   // [nnod]
-};
-
-struct BlockDev {
-    int R;               // rows (= nnod)
-    int slots, brow, crow;   // slots per row and the row lengths (brow_of, crow_of)
-    const int *perm;     // row -> node
-    const int *nslot;    // [R]
-    const int *bcol;     // [R][crow] column node of each slot; [slots] = nslot
-    const unsigned long long *bloc;   // [R][crow][nbw] byte k: local index of the column node
-                                      // in the k-th adjacent element of the row node (0xFF: absent)
-    int nbw;             // words of bloc per slot: ceil(elements per node / 8)
-    double *blk;         // [R][brow]: value (r, c) of slot s at (r*3+c)*slots + s
-    float *blk32;        // FP32 copy of blk (tuned mode), or null
-    __host__ __device__ size_t si(int p, int s) const { return (size_t)p * crow + s; }
-    __host__ __device__ size_t bi(int p, int s, int q) const { return (size_t)p * brow + (size_t)q * slots + s; }
-};
-
-// The items of a constitutive pass, entry t of the launch order (`order`,
-// or the natural order when it is null).  With a device queue (`queue`
-// non-null, a persistent grid) every warp takes the next 32 entries until
-// the order is exhausted, so the work-sorted order is served heaviest first
-// and no CTA slot idles behind one slow warp; otherwise thread t takes
-// entry t.
-template <typename F>
-__device__ __forceinline__ void for_each_item(int n, const int *__restrict__ order, int *queue, F &&f)
-{
-    if (queue) {
-        const int lane = threadIdx.x & 31;
-        for (;;) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(queue, 32);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base >= n) return;
-            const int t = base + lane;
-            if (t < n) f(order ? order[t] : t);
-        }
-    }
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) f(order ? order[t] : t);
-}
-
-// ---------------------------------------------------------------- element pass
-// ELVALS per element (src/fasolt/Elvals.f90:31-126): gather, SHAPE_12,
-// DSTRNS, DSTRSS, store the GP increments and the element record.
-template <int NS>
-__global__ void __launch_bounds__(128) k_elem(MeshDev Mh, DevMat M, DevCtrl C, DevGp G,
-                                              const double *__restrict__ x,
-                                              const double *__restrict__ dx, double *rec,
-                                              double dt, int inc, int nit,
-                                              unsigned long long *errkey, const int *__restrict__ order,
-                                              int *queue)
-{
-#if FAS_SMEM_TABLES
-    extern __shared__ double s_tables[];
-    if (M.stage_t > 0) M = stage_tables(M, s_tables);
-#endif
-    for_each_item(Mh.nlmnt, order, queue, [&](int e) {
-        if (Mh.lt[e] < 9) return;   // tie element: no Gauss point
-        const int ne = Mh.nlmnt;
-        double xl[8][3], dxl[8][3];
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            const int n = Mh.ln[a * ne + e];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                xl[a][c] = x[3 * n + c];
-                dxl[a][c] = dx[3 * n + c];
-            }
-        }
-        double sfd[8][3];
-        const double w = shape12(xl, sfd);
-        if (w < 1.e-7) {
-            atomicMin(errkey, ((unsigned long long)e << 16) | 920ull);
-            return;
-        }
-        double del[6], r[3], defl;
-        int rc = dstrns(sfd, dxl, C.smalr, C.smale, del, r, defl);
-        if (rc) {
-            atomicMin(errkey, ((unsigned long long)e << 16) | (unsigned long long)rc);
-            return;
-        }
-        const int g = Mh.gpe[e];
-        const int ng = G.ngps;
-        double st[6], ds[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            st[k] = G.st[k * ng + g];
-            ds[k] = G.ds[k * ng + g];
-        }
-        GpOut o;
-        rc = dstrss<NS>(M, C, G, g, Mh.le[e], del, r, st, ds, dt, inc, C.nit_dev ? *C.nit_dev + 1 : nit, o);
-        if (rc) {
-            atomicMin(errkey, ((unsigned long long)e << 16) | (unsigned long long)rc);
-            return;
-        }
-        G.dep[g] = o.deff;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            G.de[k * ng + g] = del[k];
-            G.ds[k * ng + g] = ds[k];
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) G.dr[k * ng + g] = r[k];
-        double *R = rec + (size_t)e * REC;
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) R[3 * a + c] = sfd[a][c];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) R[REC_S + k] = o.t[k];
-        R[REC_W] = w;
-#pragma unroll
-        for (int i = 0; i < 6; ++i)
-#pragma unroll
-            for (int j = i; j < 6; ++j) R[REC_D + utri(i, j)] = o.chi[i][j];
-    });
-}
-
-// ELVALS per Gauss point of the quadratic elements (src/fasolt/Elvals.f90:
-// 82-126): 10-node tetrahedra with SHAPE_21 (NN 10, NPG 4,
-// src/fasolt/Shapef.f90:104-189), 20-node bricks with SHAPE_22 (20, 8,
-// :210-342) and 15-node wedges with SHAPE_23 (15, 6, :360-485); one thread
-// per (element, GP).  dnt[(g*3 + j)*NN + i] = dndn(j+1, i+1, g+1) is the
-// element type's tabulated local-derivative table and wfac its GP weight
-// factor (-0.0416667, 1, 0.16666667).  The element's nodes are streamed
-// twice -- the Jacobian, then sfd (written straight to the GP record) and
-// the displacement gradient -- so no node array is held in registers.
-// Errors are keyed by (element, GP) so the first one in the reference's
-// loop order wins.
-template <int NS, int NN, int NPG>
-__global__ void __launch_bounds__(128) k_elemq(MeshDev Mh, DevMat M, DevCtrl C, DevGp G,
-                                               const double *__restrict__ dnt, double wfac,
-                                               const double *__restrict__ x,
-                                               const double *__restrict__ dx, double *rec,
-                                               double dt, int inc, int nit,
-                                               unsigned long long *errkey, const int *__restrict__ order,
-                                               int *queue)
-{
-#if FAS_SMEM_TABLES
-    extern __shared__ double s_tables[];
-    if (M.stage_t > 0) M = stage_tables(M, s_tables);
-#endif
-    using L = RecLayout<NN>;
-    for_each_item(NPG * Mh.nlmnt, order, queue, [&](int t) {   // item e*NPG + gq
-        const int e = t / NPG, gq = t - e * NPG;
-        if (Mh.lt[e] < 9) return;   // tie element: no Gauss point
-        const int ne = Mh.nlmnt;
-        const unsigned long long key = (unsigned long long)t << 16;
-        const double *dn = dnt + gq * 3 * NN;
-        double jac[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        for (int i = 0; i < NN; ++i) {
-            const int n = Mh.ln[i * ne + e];
-            const double d0 = __ldg(dn + i), d1 = __ldg(dn + NN + i), d2 = __ldg(dn + 2 * NN + i);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double xk = x[3 * n + k];
-                jac[0][k] = jac[0][k] + d0 * xk;
-                jac[1][k] = jac[1][k] + d1 * xk;
-                jac[2][k] = jac[2][k] + d2 * xk;
-            }
-        }
-        double inv[3][3];
-        const double w = wfac * invert3(jac, inv);
-        if (w < 1.e-7) {
-            atomicMin(errkey, key | 920ull);
-            return;
-        }
-        double *R = rec + (size_t)t * L::LEN;
-        double gr[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        for (int i = 0; i < NN; ++i) {
-            const int n = Mh.ln[i * ne + e];
-            const double d0 = __ldg(dn + i), d1 = __ldg(dn + NN + i), d2 = __ldg(dn + 2 * NN + i);
-            double sf[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                sf[k] = inv[k][0] * d0 + inv[k][1] * d1 + inv[k][2] * d2;
-                R[3 * i + k] = sf[k];
-            }
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const double u = dx[3 * n + b];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) gr[a][b] = gr[a][b] + sf[a] * u;
-            }
-        }
-        double del[6], r[3], defl;
-        int rc = dstrns_grad(gr, C.smalr, C.smale, del, r, defl);
-        if (rc) {
-            atomicMin(errkey, key | (unsigned long long)rc);
-            return;
-        }
-        const int g = Mh.gpe[gq * ne + e];
-        const int ng = G.ngps;
-        double st[6], ds[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            st[k] = G.st[k * ng + g];
-            ds[k] = G.ds[k * ng + g];
-        }
-        GpOut o;
-        rc = dstrss<NS>(M, C, G, g, Mh.le[e], del, r, st, ds, dt, inc, C.nit_dev ? *C.nit_dev + 1 : nit, o);
-        if (rc) {
-            atomicMin(errkey, key | (unsigned long long)rc);
-            return;
-        }
-        G.dep[g] = o.deff;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            G.de[k * ng + g] = del[k];
-            G.ds[k * ng + g] = ds[k];
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) G.dr[k * ng + g] = r[k];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) R[L::S + k] = o.t[k];
-        R[L::W] = w;
-#pragma unroll
-        for (int i = 0; i < 6; ++i)
-#pragma unroll
-            for (int j = i; j < 6; ++j) R[L::D + utri(i, j)] = o.chi[i][j];
-    });
-}
 
 // Work-sorted launch order for the constitutive kernels: items (elements or
 // points) grouped by the operation count of their GP's last update, so the
@@ -337,176 +80,6 @@ __global__ void k_work_scatter(int n, const int *__restrict__ gp_of, const doubl
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     order[atomicAdd(&offs[work_bin(gp_of ? gp_of[i] : i, ops)], 1)] = i;
-}
-
-// Constitutive update of independent points (no mesh): DSTRSS with the
-// stored de / dr; the full tangent goes to chi[36][ngps] (column-major 6x6).
-template <int NS>
-__global__ void __launch_bounds__(128) k_points(DevMat M, DevCtrl C, DevGp G, const int *gp_iel,
-                                                double *chi, double dt, int inc, int nit,
-                                                unsigned long long *errkey, const int *__restrict__ order,
-                                                int *queue)
-{
-#if FAS_SMEM_TABLES
-    extern __shared__ double s_tables[];
-    if (M.stage_t > 0) M = stage_tables(M, s_tables);
-#endif
-    for_each_item(G.ngps, order, queue, [&](int g) {
-        const int ng = G.ngps;
-        double de[6], r[3], st[6], ds[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            de[k] = G.de[k * ng + g];
-            st[k] = G.st[k * ng + g];
-            ds[k] = G.ds[k * ng + g];
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) r[k] = G.dr[k * ng + g];
-        GpOut o;
-        const int rc = dstrss<NS>(M, C, G, g, gp_iel[g], de, r, st, ds, dt, inc, nit, o);
-        if (rc) {
-            atomicMin(errkey, ((unsigned long long)g << 16) | (unsigned long long)rc);
-            return;
-        }
-        G.dep[g] = o.deff;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) G.ds[k * ng + g] = ds[k];
-#pragma unroll
-        for (int i = 0; i < 6; ++i)
-#pragma unroll
-            for (int j = 0; j < 6; ++j) chi[(i + 6 * j) * (size_t)ng + g] = o.chi[i][j];
-    });
-}
-
-// ---------------------------------------------------------------- warp-cooperative pass
-// ELVALS per element with one warp per element: every lane forms the
-// element kinematics (identical values), the warp runs dstrss_wc with lane i
-// owning slip system i, and the lanes share out the stores.
-template <int NA>
-__global__ void __launch_bounds__(128) k_elem_wc(MeshDev Mh, DevMat M, DevCtrl C, DevGp G,
-                                                 const double *__restrict__ x,
-                                                 const double *__restrict__ dx, double *rec,
-                                                 double dt, int inc, int nit,
-                                                 unsigned long long *errkey)
-{
-    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (e >= Mh.nlmnt) return;           // whole warps only
-    if (Mh.lt[e] < 9) return;            // tie element: no Gauss point
-    const int ne = Mh.nlmnt;
-    double del[6], r[3], defl;
-    double *R = rec + (size_t)e * REC;
-    {
-        double xl[8][3], dxl[8][3];
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            const int n = Mh.ln[a * ne + e];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                xl[a][c] = x[3 * n + c];
-                dxl[a][c] = dx[3 * n + c];
-            }
-        }
-        double sfd[8][3];
-        const double w = shape12(xl, sfd);
-        if (w < 1.e-7) {
-            if (lane == 0) atomicMin(errkey, ((unsigned long long)e << 16) | 920ull);
-            return;
-        }
-        const int rc = dstrns(sfd, dxl, C.smalr, C.smale, del, r, defl);
-        if (rc) {
-            if (lane == 0) atomicMin(errkey, ((unsigned long long)e << 16) | (unsigned long long)rc);
-            return;
-        }
-        // record: lanes 0-23 shape derivatives, lane 30 the weight
-        double v = 0.0;
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                if (lane == 3 * a + c) v = sfd[a][c];
-        if (lane == REC_W) v = w;
-        if (lane < 24 || lane == REC_W) R[lane] = v;
-    }
-    const int g = Mh.gpe[e];
-    const int ng = G.ngps;
-    double st[6], ds[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        st[k] = G.st[k * ng + g];
-        ds[k] = G.ds[k * ng + g];
-    }
-    wc::GpOutW o;
-    const int rc = wc::dstrss_wc<NA>(M, C, G, g, Mh.le[e], del, r, st, ds, dt, inc,
-                                     C.nit_dev ? *C.nit_dev + 1 : nit, o);
-    if (rc) {
-        if (lane == 0) atomicMin(errkey, ((unsigned long long)e << 16) | (unsigned long long)rc);
-        return;
-    }
-    if (lane == 0) G.dep[g] = o.deff;
-    if (lane < 6) {
-        double dk = 0.0, sk = 0.0, tk = 0.0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-            if (k == lane) {
-                dk = del[k];
-                sk = ds[k];
-                tk = o.t[k];
-            }
-        G.de[lane * ng + g] = dk;
-        G.ds[lane * ng + g] = sk;
-        R[REC_S + lane] = tk;
-        // tangent upper triangle, row `lane`
-#pragma unroll
-        for (int j = 0; j < 6; ++j)
-            if (j >= lane) R[REC_D + utri(lane, j)] = o.chirow[j];
-    }
-    if (lane < 3) {
-        double rk = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (k == lane) rk = r[k];
-        G.dr[lane * ng + g] = rk;
-    }
-}
-
-// Independent points with one warp per point (the micro-benchmark path).
-template <int NA>
-__global__ void __launch_bounds__(128) k_points_wc(DevMat M, DevCtrl C, DevGp G, const int *gp_iel,
-                                                   double *chi, double dt, int inc, int nit,
-                                                   unsigned long long *errkey)
-{
-    const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (g >= G.ngps) return;
-    const int ng = G.ngps;
-    double de[6], r[3], st[6], ds[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        de[k] = G.de[k * ng + g];
-        st[k] = G.st[k * ng + g];
-        ds[k] = G.ds[k * ng + g];
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) r[k] = G.dr[k * ng + g];
-    wc::GpOutW o;
-    const int rc = wc::dstrss_wc<NA>(M, C, G, g, gp_iel[g], de, r, st, ds, dt, inc, nit, o);
-    if (rc) {
-        if (lane == 0) atomicMin(errkey, ((unsigned long long)g << 16) | (unsigned long long)rc);
-        return;
-    }
-    if (lane == 0) G.dep[g] = o.deff;
-    if (lane < 6) {
-        double sk = 0.0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-            if (k == lane) sk = ds[k];
-        G.ds[lane * ng + g] = sk;
-    }
-    if (lane < 6) {   // row `lane` of the tangent, column-major 6x6 per point
-#pragma unroll
-        for (int j = 0; j < 6; ++j) chi[(size_t)(lane + 6 * j) * ng + g] = o.chirow[j];
-    }
 }
 
 // gaussm (src/fasolt/Elvals.f90:132-220) for node pair (i, j) of one
@@ -1717,9 +1290,13 @@ __global__ void __launch_bounds__(NT) k_sor_small(BlockDev B, const int *__restr
 // ---------------------------------------------------------------- FP32 SOR refinement
 // FP64 residual of the assembled system, r = rhs - K x, one warp per row.
 // Skipped once the solve has converged.
+// With `ext` (the persistent solve) the residual and the iterate also go to
+// the extras of the node's row, ext + eoff[node] (right-hand side first, base
+// from the seventh double).
 __global__ void __launch_bounds__(256) k_residual(BlockDev B, const double *__restrict__ rhs,
                                                   const double *__restrict__ x, double *r,
-                                                  const SorCtl *ctl)
+                                                  const SorCtl *ctl, double *ext = nullptr,
+                                                  const unsigned *__restrict__ eoff = nullptr)
 {
     if (((volatile const SorCtl *)ctl)->conv) return;
     const int lane = threadIdx.x & 31;
@@ -1747,6 +1324,15 @@ __global__ void __launch_bounds__(256) k_residual(BlockDev B, const double *__re
             r[3 * n] = rhs[3 * n] - a0;
             r[3 * n + 1] = rhs[3 * n + 1] - a1;
             r[3 * n + 2] = rhs[3 * n + 2] - a2;
+            if (ext) {
+                double *e = ext + eoff[n];
+                e[0] = rhs[3 * n] - a0;
+                e[1] = rhs[3 * n + 1] - a1;
+                e[2] = rhs[3 * n + 2] - a2;
+                e[6] = x[3 * n];
+                e[7] = x[3 * n + 1];
+                e[8] = x[3 * n + 2];
+            }
         }
     }
 }

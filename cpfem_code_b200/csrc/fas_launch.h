@@ -1,0 +1,35 @@
+// fas_launch.h -- kernels that live in their own translation units (they take
+// minutes to compile): host code takes their launch handles from here.
+#pragma once
+
+#include "fas_adjoint_types.cuh"
+#include "fas_device.cuh"
+#include "fas_layout.cuh"
+
+namespace fasdev {
+
+using ElemFn = void (*)(MeshDev, DevMat, DevCtrl, DevGp, const double *, const double *, double *, double, int, int,
+                        unsigned long long *, const int *, int *);
+using ElemqFn = void (*)(MeshDev, DevMat, DevCtrl, DevGp, const double *, double, const double *, const double *,
+                         double *, double, int, int, unsigned long long *, const int *, int *);
+using ElemWcFn = void (*)(MeshDev, DevMat, DevCtrl, DevGp, const double *, const double *, double *, double, int, int,
+                          unsigned long long *);
+using PointsFn = void (*)(DevMat, DevCtrl, DevGp, const int *, double *, double, int, int, unsigned long long *,
+                          const int *, int *);
+using PointsWcFn = void (*)(DevMat, DevCtrl, DevGp, const int *, double *, double, int, int, unsigned long long *);
+using ReplayFwdFn = void (*)(DevMat, DevCtrl, DevGp, const int *, const double *, ReplayDev, double *, double *, int,
+                             double *, double *, unsigned long long *);
+using ReplayAdjFn = void (*)(DevMat, DevCtrl, DevGp, const int *, ReplayDev, const double *, double *, int, double *,
+                             double *, double *, double *, unsigned long long *);
+
+// ns: the compile-time bound on slip systems (12, 32 or 60; 12 or 32 for
+// the warp and replay kernels); nn: nodes of a quadratic element (10, 15, 20)
+ElemFn elem_kernel(int ns);
+ElemqFn elemq_kernel(int ns, int nn);
+ElemWcFn elem_wc_kernel(int ns);
+PointsFn points_kernel(int ns);
+PointsWcFn points_wc_kernel(int ns);
+ReplayFwdFn replay_fwd_kernel(int ns);
+ReplayAdjFn replay_adj_kernel(int ns);
+
+}  // namespace fasdev

@@ -64,9 +64,10 @@ extern "C" {
 #define FAS_MODE_CP_WARP      8u  /* Gauss-point update with one warp per GP
                                      (lanes = slip systems) instead of one
                                      thread per GP; at most 32 systems      */
-#define FAS_MODE_SOR_GRID     4u  /* always use the grid-wide SOR launches,
-                                     also for meshes small enough for the
-                                     one-CTA solve                          */
+#define FAS_MODE_SOR_GRID     4u  /* the FP32 form also on meshes of at most
+                                     256 nodes (512 with 20-node rows), which
+                                     solve in FP64 otherwise; and the grid-wide
+                                     launches of fas_gpu_facsls_noalloc there */
 #define FAS_MODE_TANGENT_CONSISTENT 32u  /* element tangent (B X^-1 B^T + S)^-1
                                      of the local system re-evaluated at
                                      the converged stress (the implicit-
@@ -83,12 +84,13 @@ extern "C" {
                                      materials differ in their slip-system
                                      counts (mixed FCC/HCP) take the queue
                                      without the flag                       */
-#define FAS_MODE_SOR_TILES   16u  /* grid-wide SOR as one persistent launch
-                                     per solve: spatial tiles of rows, one
-                                     per SM, that start each colour once
-                                     their neighbour tiles have finished the
-                                     previous one (8-node bricks; other
-                                     meshes keep one launch per colour)     */
+#define FAS_MODE_SOR_TILES   16u  /* accepted for callers of earlier versions, where
+                                     it chose the solve as one persistent
+                                     launch over spatial tiles: every solve
+                                     runs so now (a mesh too large for the
+                                     tiles' shared memory, or of more than 64
+                                     colours, and FAS_MODE_SOR_SYM keep one
+                                     launch per colour)                     */
 #define FAS_MODE_GRAPH      128u  /* fas_gpu_nriter as one CUDA graph per
                                      increment: the Newton loop and the SOR
                                      loop are conditional while nodes whose
@@ -101,9 +103,8 @@ extern "C" {
                                      same results to the bit; combines with
                                      FAS_MODE_SOR_FP32 (cycles of sweeps,
                                      fold and residual as the loop body).
-                                     With FAS_MODE_SOR_TILES, and while
-                                     profiling with prof >= 2, the host loop
-                                     runs.  The graph of an increment is
+                                     While profiling with prof >= 2 the host
+                                     loop runs.  The graph of an increment is
                                      built on its first call and kept until
                                      the mode changes                       */
 #define FAS_MODE_SOR_SYM    256u  /* with FAS_MODE_SOR_FP32 on 8-node meshes:
@@ -393,17 +394,17 @@ FAS_API int32_t fas_gpu_profile(fas_handle *h, int32_t enable, fas_profile *out)
  * Who needs it: a driver that must not allocate device memory once set-up
  * is over -- one that hands all memory left after fas_gpu_create to
  * another allocator (a coupled solver's pool, a caching allocator) or runs
- * under a fixed device-memory cap.  fas_gpu_facsls allocates on first use
- * (it instantiates a CUDA graph of its sweeps), which can then fail in
- * the middle of a run; this entry point never does.
+ * under a fixed device-memory cap.  fas_gpu_facsls allocates on the first
+ * use of a value type that the handle's first mode does not use, which can
+ * then fail in the middle of a run; this entry point never does.
  *
- * What it does: the same solve as fas_gpu_facsls -- the same iterates
- * (one launch per colour, the colour order, the reciprocal-diagonal
- * quotients), sweep count and stopping test, same return codes (903, 904,
+ * What it does: the same solve as fas_gpu_facsls -- the same iteration in
+ * the same colour order with one launch per colour (iterates equal to
+ * rounding), sweep count and stopping test, same return codes (903, 904,
  * FAS_E_TIMEOUT) -- on the FP64 blocks, with the kernels' scratch (the
  * stopping-test control words and one pair of partial sums per colour
  * CTA) in a static device array of this library instead of buffers of the
- * handle.  It ignores FAS_MODE_SOR_FP32 and FAS_MODE_SOR_TILES and is not
+ * handle.  It ignores FAS_MODE_SOR_FP32 and is not
  * timed by fas_gpu_profile.  It reads the stopping flag between chunks of
  * sweeps, so it synchronises the handle's stream before it returns.
  *
