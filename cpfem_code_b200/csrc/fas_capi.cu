@@ -194,6 +194,16 @@ struct fas_handle {
     int sor_nblk_tot = 0, sor_nblk_tot32 = 0, nr_nblk = 0;
     DVec<double> part_sor, part_nr, sums;
     bool mixed_phases = false;   // GPs of materials with different slip-system counts
+    // the group pass (k_cp): whether every GP's material qualifies, and its
+    // lists by the bound on the slip systems
+    struct CpClass {
+        int ns = 0, n = 0;       // the bound, and the GPs of the class
+        unsigned grid = 0;       // CTAs that reside at once
+        DVec<int> list;
+    };
+    DVec<double> cp_w;
+    bool cp_group = false;
+    CpClass cp_class[3];
     size_t stage_bytes = 0;      // shared memory of the constitutive kernels' table copy
     DVec<unsigned long long> ekey;
     DVec<int> flags;
@@ -1004,13 +1014,13 @@ int create_impl(fas_handle *h, const fas_mesh_desc *Md, const fas_matl_desc *T, 
                 nel[(size_t)k * h->nnod + n] = h->ne_locl[h->ne_ptr[n] + k];
             }
         }
+        CKA(h->gp_item.alloc(h->h_gpe.size()));
+        CK(h->gp_item.put(h->h_gpe.data(), h->h_gpe.size(), s));
         if (NN != 8) {
             const std::vector<double> t = NN == 20 ? shape22_table() : (NN == 10 ? shape21_table() : shape23_table());
             h->wfac = NN == 20 ? 1.0 : (NN == 10 ? -0.0416667 : 0.16666667);
             CKA(h->dnq.alloc(t.size()));
             CK(h->dnq.put(t.data(), t.size(), s));
-            CKA(h->gp_item.alloc(h->h_gpe.size()));
-            CK(h->gp_item.put(h->h_gpe.data(), h->h_gpe.size(), s));
         }
         CKA(h->ln.alloc(lnT.size()));
         CKA(h->gpe.alloc(gpeT.size()));
@@ -1075,6 +1085,38 @@ int create_impl(fas_handle *h, const fas_mesh_desc *Md, const fas_matl_desc *T, 
         ns_used = ns_used == 0 ? ns : (ns_used == ns ? ns : -1);
     }
     h->mixed_phases = ns_used < 0;
+    // the group pass serves materials with one latent hardening number q and
+    // self hardening not below it, positive rate exponents and hardening
+    // coefficients not below zero: what its formula needs (fas_cp_group.cuh).
+    // It is faster at every size (27 points 0.07 against 0.61 ms, 2^20 points 11.6
+    // against 28.2 ms), so that size does not enter the rule
+    std::vector<char> one(nm, 1);
+    for (int m = 0; m < nm; ++m) {
+        const int ns = h->M.ns[m];
+        const double *S = &sm[(size_t)m * MAXSS * MAXSS];
+        const double q = ns > 1 ? S[1] : 0.0;
+        bool ok = q >= 0.0;
+        for (int i = 0; i < ns && ok; ++i) {
+            const double *a = &ampar[((size_t)m * MAXSS + i) * 6];
+            ok = a[0] > 0.0 && a[1] >= 0.0 && a[2] >= 0.0;
+            for (int j = 0; j < ns && ok; ++j) ok = i == j ? S[i * ns + j] >= q : S[i * ns + j] == q;
+        }
+        one[m] = ok;
+        h->M.hq[m] = q;
+    }
+    h->cp_group = true;
+    for (int g = 0; g < h->ngps && h->cp_group; ++g) h->cp_group = one[std::abs(h->h_gp_iel[g]) - 1];
+    if (h->cp_group) {
+        const int bound[3] = {12, 32, 60};
+        const int nitem = h->point_mode ? h->ngps : (int)h->h_gpe.size();
+        for (int t = 0; t < nitem; ++t) {
+            const int g = h->point_mode ? t : h->h_gpe[t];
+            if (g < 0) continue;                     // a tie element's places
+            const int ns = h->M.ns[std::abs(h->h_gp_iel[g]) - 1];
+            ++h->cp_class[ns <= 12 ? 0 : ns <= 32 ? 1 : 2].n;
+        }
+        for (int c = 0; c < 3; ++c) h->cp_class[c].ns = bound[c];
+    }
     h->ns_tmpl = h->maxns <= 12 ? 12 : (h->maxns <= 32 ? 32 : 60);
     // tables in shared memory (FAS_SMEM_TABLES builds) when they fit the
     // default 48 KB of a launch
@@ -1206,6 +1248,7 @@ int down_field(fas_handle *h, void *dst, int rb, int ld, int nk, int n, const do
 }
 
 int prepare_solve(fas_handle *h);
+int ensure_group(fas_handle *h);
 
 int upload_impl(fas_handle *h, const fas_state_desc *S)
 {
@@ -1249,6 +1292,7 @@ int upload_impl(fas_handle *h, const fas_state_desc *S)
         if (!rc) rc = prepare_solve(h);
         if (rc) return rc;
     }
+    if (!h->have_state && (rc = ensure_group(h))) return rc;
     CK(cudaStreamSynchronize(h->stream));
     h->have_state = true;
     return 0;
@@ -1334,10 +1378,89 @@ template <typename K> unsigned cp_grid(fas_handle *h, K kern, long long n, int *
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, *bs, h->stage_bytes) != cudaSuccess || occ < 1)
         return full;
-    if (!h->cp_queue.p && h->cp_queue.alloc(1) != cudaSuccess) return full;
+    if (!h->cp_queue.p && h->cp_queue.alloc(8) != cudaSuccess) return full;
     if (cudaMemsetAsync(h->cp_queue.p, 0, sizeof(int), h->stream) != cudaSuccess) return full;
     *queue = h->cp_queue.p;
     return std::min<unsigned>(full, (unsigned)occ * (unsigned)h->nsm);
+}
+
+// Whether the pass runs with a group of lanes per GP (k_cp): the materials
+// allow it and no mode asks for another form.
+bool group_pass(const fas_handle *h)
+{
+    return h->cp_group && !(h->mode & (FAS_MODE_CP_WARP | FAS_MODE_CP_QUEUE | FAS_MODE_TANGENT_CONSISTENT));
+}
+
+// Scratch and lists of the group pass, allocated with the handle's state.  A
+// handle whose GPs leave no room for them (344 bytes a GP) keeps the general
+// kernels.
+int ensure_group(fas_handle *h)
+{
+    if (!group_pass(h)) return 0;
+    cudaError_t e = cudaSuccess;
+    if (!h->cp_w.p) e = h->cp_w.alloc(CPW * (size_t)h->ngps);
+    if (e == cudaSuccess && !h->cp_queue.p) e = h->cp_queue.alloc(8);
+    for (auto &c : h->cp_class)
+        if (e == cudaSuccess && c.n > 0 && !c.list.p) e = c.list.alloc(c.n);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        h->cp_w.release();
+        for (auto &c : h->cp_class) c.list.release();
+        h->cp_group = false;
+        return 0;
+    }
+    CKA(e);
+    return 0;
+}
+
+CpWork group_work(fas_handle *h)
+{
+    CpWork w;
+    w.w = h->cp_w.p;
+    w.chi = h->chi_pts.p;
+    w.count = h->cp_queue.p;
+    w.head = h->cp_queue.p + 4;
+    for (int k = 0; k < 3; ++k) w.list[k] = h->cp_class[k].list.p;
+    w.rec = h->point_mode ? nullptr : h->rec.p;
+    w.reclen = 3 * h->nn + 32;
+    w.off_s = 3 * h->nn;
+    w.gp_of = h->point_mode ? nullptr : h->gp_item.p;
+    w.gp_iel = h->gp_iel.p;
+    return w;
+}
+
+// DSTRSS of every GP by the group pass: kinematics and what a point does once,
+// the iterations by bound on the slip systems (on as many CTAs as reside at
+// once), the tangents.
+int launch_group(fas_handle *h, double dt, int inc, int nit)
+{
+    cudaStream_t s = h->stream;
+    CK(cudaMemsetAsync(h->cp_queue.p, 0, 8 * sizeof(int), s));
+    const CpWork W = group_work(h);
+    if (h->point_mode)
+        prep_points_kernel()<<<nblocks(h->ngps, 128), 128, 0, s>>>(h->M, h->gp(), W);
+    else if (h->nn == 8)
+        prep8_kernel()<<<nblocks(h->nlmnt, 128), 128, 0, s>>>(h->mesh(), h->M, h->C, h->gp(), W, h->x.p, h->dx.p, h->ekey.p);
+    else
+        prepq_kernel(h->nn)<<<nblocks((long long)h->npg * h->nlmnt, 128), 128, 0, s>>>(
+            h->mesh(), h->M, h->C, h->gp(), W, h->dnq.p, h->wfac, h->x.p, h->dx.p, h->ekey.p);
+    LAUNCHED(h);
+    for (int k = 0; k < 3; ++k) {
+        auto &c = h->cp_class[k];
+        if (c.n == 0) continue;
+        const auto kern = cp_kernel(c.ns);
+        if (c.grid == 0) {
+            int occ = 0;
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, CP_THREADS, 0));
+            c.grid = std::max(occ, 1) * h->nsm;
+        }
+        const unsigned blk = std::min<unsigned>(c.grid, nblocks((long long)c.n * cp_lanes(c.ns), CP_THREADS));
+        kern<<<blk, CP_THREADS, 0, s>>>(h->M, h->C, h->gp(), W, k, dt, inc, nit, h->ekey.p);
+        LAUNCHED(h);
+        cp_tangent_kernel()<<<nblocks(c.n, 128), 128, 0, s>>>(h->gp(), W, k);
+        LAUNCHED(h);
+    }
+    return 0;
 }
 
 int launch_elem(fas_handle *h, int inc, int nit)
@@ -1346,7 +1469,11 @@ int launch_elem(fas_handle *h, int inc, int nit)
     const int ns = h->ns_tmpl;
     const double dt = h->h_tiem[inc - 1];
     int *queue = nullptr, bs = 128;
-    if (h->nn != 8) {   // quadratic elements: one thread per (element, GP)
+    if (int rc = ensure_group(h)) return rc;
+    const bool group = group_pass(h);
+    if (group) {
+        if (int rc = launch_group(h, dt, inc, nit)) return rc;
+    } else if (h->nn != 8) {   // quadratic elements: one thread per (element, GP)
         const auto kern = elemq_kernel(ns, h->nn);
         const long long items = (long long)h->npg * h->nlmnt;
         const int *order = work_order(h, (int)items, h->gp_item.p);
@@ -1365,7 +1492,7 @@ int launch_elem(fas_handle *h, int inc, int nit)
     }
     sp.end();
     keep(h, sp);
-    LAUNCHED(h);
+    if (!group) LAUNCHED(h);
     h->P.n_constitutive++;
     h->P.gp_updates += h->ngps;
     return 0;
@@ -2194,7 +2321,7 @@ int ensure_inc_graph(fas_handle *h, int inc, cudaGraphExec_t *out)
     if (!h->cap3) CK(cudaStreamCreateWithFlags(&h->cap3, cudaStreamNonBlocking));
     if (!h->nrdev.p) CKA(h->nrdev.alloc(1));
     if (!h->nrrep.p) CKA(h->nrrep.alloc((size_t)std::max(h->C.maxit, 1)));
-    if (!h->cp_queue.p) CKA(h->cp_queue.alloc(1));
+    if (!h->cp_queue.p) CKA(h->cp_queue.alloc(8));
     if (int rc = ensure_fp32(h)) return rc;
     if (int rc = ensure_sym(h)) return rc;
     const bool fp32 = graph_fp32(h);
@@ -2202,7 +2329,9 @@ int ensure_inc_graph(fas_handle *h, int inc, cudaGraphExec_t *out)
     // the solve's and the work order's buffers are sized outside the capture
     if (flow_on(h, fp32))
         if (int rc = fp32 ? ensure_flow<float>(h) : ensure_flow<double>(h)) return rc;
-    if (h->nn != 8)
+    if (int rc = ensure_group(h)) return rc;
+    if (group_pass(h)) {
+    } else if (h->nn != 8)
         work_order(h, h->npg * h->nlmnt, h->gp_item.p);
     else if (!(h->mode & FAS_MODE_CP_WARP))
         work_order(h, h->nlmnt, h->gpe.p);
@@ -2664,7 +2793,11 @@ int32_t fas_gpu_constitutive(fas_handle *h, int32_t inc, int32_t nit)
     CK(cudaMemsetAsync(h->ekey.p, 0xFF, sizeof(unsigned long long), s));
     Span sp(h, &h->P.ms_constitutive);
     const double dt = h->h_tiem[inc - 1];
-    if ((h->mode & FAS_MODE_CP_WARP) && h->maxns <= 32) {
+    if (int rc = ensure_group(h)) return rc;
+    const bool group = group_pass(h) && h->point_mode;
+    if (group) {
+        if (int rc = launch_group(h, dt, inc, nit)) return rc;
+    } else if ((h->mode & FAS_MODE_CP_WARP) && h->maxns <= 32) {
         points_wc_kernel(h->ns_tmpl)<<<nblocks(32LL * h->ngps, 128), 128, 0, s>>>(
             h->M, h->C, h->gp(), h->gp_iel.p, h->chi_pts.p, dt, inc, nit, h->ekey.p);
     } else {
@@ -2677,7 +2810,7 @@ int32_t fas_gpu_constitutive(fas_handle *h, int32_t inc, int32_t nit)
     }
     sp.end();
     keep(h, sp);
-    LAUNCHED(h);
+    if (!group) LAUNCHED(h);
     h->P.n_constitutive++;
     h->P.gp_updates += h->ngps;
     CK(cudaMemcpyAsync(h->hc->ekey, h->ekey.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));

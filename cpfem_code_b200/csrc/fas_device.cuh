@@ -24,6 +24,7 @@ struct DevMat {
     int nmatl;
     int ns[12];
     double amax[12];            // MAXVAL(ampar(1,1:ns)) per material (SLPFTA conv)
+    double hq[12];              // smatrx(i, j) for i /= j where it is one number (fas_cp_group.cuh)
     const double *e;            // [nmatl][9]
     const double *ssang;        // [nmatl][60]
     const double *ab, *an;      // [nmatl][60][3]

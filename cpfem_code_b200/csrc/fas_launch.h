@@ -3,6 +3,7 @@
 #pragma once
 
 #include "fas_adjoint_types.cuh"
+#include "fas_cp_types.h"
 #include "fas_device.cuh"
 #include "fas_layout.cuh"
 
@@ -17,6 +18,12 @@ using ElemWcFn = void (*)(MeshDev, DevMat, DevCtrl, DevGp, const double *, const
 using PointsFn = void (*)(DevMat, DevCtrl, DevGp, const int *, double *, double, int, int, unsigned long long *,
                           const int *, int *);
 using PointsWcFn = void (*)(DevMat, DevCtrl, DevGp, const int *, double *, double, int, int, unsigned long long *);
+using CpFn = void (*)(DevMat, DevCtrl, DevGp, CpWork, int, double, int, int, unsigned long long *);
+using CpTangentFn = void (*)(DevGp, CpWork, int);
+using PrepPointsFn = void (*)(DevMat, DevGp, CpWork);
+using Prep8Fn = void (*)(MeshDev, DevMat, DevCtrl, DevGp, CpWork, const double *, const double *, unsigned long long *);
+using PrepqFn = void (*)(MeshDev, DevMat, DevCtrl, DevGp, CpWork, const double *, double, const double *, const double *,
+                         unsigned long long *);
 using ReplayFwdFn = void (*)(DevMat, DevCtrl, DevGp, const int *, const double *, ReplayDev, double *, double *, int,
                              double *, double *, unsigned long long *);
 using ReplayAdjFn = void (*)(DevMat, DevCtrl, DevGp, const int *, ReplayDev, const double *, double *, int, double *,
@@ -29,6 +36,12 @@ ElemqFn elemq_kernel(int ns, int nn);
 ElemWcFn elem_wc_kernel(int ns);
 PointsFn points_kernel(int ns);
 PointsWcFn points_wc_kernel(int ns);
+CpFn cp_kernel(int ns);      // the group pass (CTAs of CP_THREADS), ns as above
+int cp_lanes(int ns);        // its lanes per Gauss point
+CpTangentFn cp_tangent_kernel();
+PrepPointsFn prep_points_kernel();
+Prep8Fn prep8_kernel();
+PrepqFn prepq_kernel(int nn);
 ReplayFwdFn replay_fwd_kernel(int ns);
 ReplayAdjFn replay_adj_kernel(int ns);
 

@@ -62,8 +62,9 @@ extern "C" {
                                      residual every 16 sweeps               */
 #define FAS_MODE_SOR_NATURAL  2u  /* (oracle only) natural-order SOR        */
 #define FAS_MODE_CP_WARP      8u  /* Gauss-point update with one warp per GP
-                                     (lanes = slip systems) instead of one
-                                     thread per GP; at most 32 systems      */
+                                     (lanes = slip systems) instead of the
+                                     default's 4, 8 or 16 lanes; at most 32
+                                     systems                                */
 #define FAS_MODE_SOR_GRID     4u  /* the FP32 form also on meshes of at most
                                      256 nodes (512 with 20-node rows), which
                                      solve in FP64 otherwise; and the grid-wide
@@ -79,11 +80,12 @@ extern "C" {
 #define FAS_MODE_CP_QUEUE    64u  /* constitutive passes on a persistent grid
                                      whose warps take the next 32 GPs of the
                                      work-sorted (heaviest first) order from
-                                     a device queue, instead of one thread
-                                     per GP in that order.  Meshes whose GPs'
-                                     materials differ in their slip-system
-                                     counts (mixed FCC/HCP) take the queue
-                                     without the flag                       */
+                                     a device queue, with one thread per GP.
+                                     Without the flag materials with one
+                                     latent hardening number run with a group
+                                     of lanes per GP; others run with one
+                                     thread per GP in that order, by the
+                                     queue if their slip-system counts differ */
 #define FAS_MODE_SOR_TILES   16u  /* accepted for callers of earlier versions, where
                                      it chose the solve as one persistent
                                      launch over spatial tiles: every solve
