@@ -1388,7 +1388,7 @@ template <typename K> unsigned cp_grid(fas_handle *h, K kern, long long n, int *
 // allow it and no mode asks for another form.
 bool group_pass(const fas_handle *h)
 {
-    return h->cp_group && !(h->mode & (FAS_MODE_CP_WARP | FAS_MODE_CP_QUEUE | FAS_MODE_TANGENT_CONSISTENT));
+    return h->cp_group && !(h->mode & (FAS_MODE_CP_WARP | FAS_MODE_TANGENT_CONSISTENT));
 }
 
 // Scratch and lists of the group pass, allocated with the handle's state.  A

@@ -77,15 +77,17 @@ extern "C" {
                                      reference) instead of CPSTRS's chi of
                                      the last iterate (Cpstrs.f90:154-162);
                                      symmetrised like chi                  */
-#define FAS_MODE_CP_QUEUE    64u  /* constitutive passes on a persistent grid
-                                     whose warps take the next 32 GPs of the
-                                     work-sorted (heaviest first) order from
-                                     a device queue, with one thread per GP.
-                                     Without the flag materials with one
-                                     latent hardening number run with a group
-                                     of lanes per GP; others run with one
-                                     thread per GP in that order, by the
-                                     queue if their slip-system counts differ */
+#define FAS_MODE_CP_QUEUE    64u  /* constitutive passes with one thread per
+                                     GP on a persistent grid whose warps take
+                                     the next 32 GPs of the work-sorted
+                                     (heaviest first) order from a device
+                                     queue, instead of a thread per GP in that
+                                     order; meshes whose GPs' materials differ
+                                     in their slip-system counts do so without
+                                     the flag.  Materials with one latent
+                                     hardening number run with a group of
+                                     lanes per GP from a device queue, with
+                                     and without the flag                   */
 #define FAS_MODE_SOR_TILES   16u  /* accepted for callers of earlier versions, where
                                      it chose the solve as one persistent
                                      launch over spatial tiles: every solve
