@@ -18,9 +18,10 @@ import tempfile
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "lib", "libfasgpu.so")
-SOURCES = ["fas_capi.cu", "fas_cp.cu", "fas_cpq.cu", "fas_cpg.cu", "fas_adj.cu"]
-DEPS = SOURCES + ["fas_kernels.cuh", "fas_layout.cuh", "fas_cp.cuh", "fas_cp_group.cuh", "fas_sor_flow.cuh", "fas_device_warp.cuh",
-                  "fas_adjoint.cuh", "fas_adjoint_types.cuh", "fas_device.cuh", "fas_launch.h", "fas_cp_types.h", "fas_flops.h", "fas_rng.h"]
+SOURCES = ["fas_capi.cu", "fas_cp.cu", "fas_cpq.cu", "fas_cpg.cu", "fas_adj.cu", "fas_adjg.cu"]
+DEPS = SOURCES + ["fas_kernels.cuh", "fas_layout.cuh", "fas_cp.cuh", "fas_cp_math.cuh", "fas_cp_group.cuh", "fas_sor_flow.cuh",
+                  "fas_device_warp.cuh", "fas_adjoint.cuh", "fas_replay_group.cuh", "fas_adjoint_types.cuh", "fas_device.cuh", "fas_launch.h",
+                  "fas_cp_types.h", "fas_flops.h", "fas_rng.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 TUNED = os.path.join(HERE, "tuned.json")
 

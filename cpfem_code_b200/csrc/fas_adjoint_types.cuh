@@ -16,4 +16,12 @@ struct ReplayDev {
     int zs;          // stride (in rows of ngps) of one state record: 9 + the widest ns
 };
 
+// Rows of one increment's record (k_replay_adj's layout) from `rec`, or null.
+struct ReplayRows {
+    double *commit, *next;       // records of the increment committed and of the one prepared
+    double *chk;                 // checkpoint rows to write, or null
+    const double *load;          // checkpoint rows to start from, or null
+    int flag;                    // row of the branch in a record
+};
+
 }  // namespace fasdev

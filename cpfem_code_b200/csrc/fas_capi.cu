@@ -99,6 +99,8 @@ struct ReplayBufs {
     DVec<double> de, dr, dt, w, y, chk, rec;
     DVec<double> sv, dsv, srate, erepmd, ops, jg, eq, gst, gsv, gp;
     DVec<int> twinsys, timestwinned, cp_iters, tflag;
+    DVec<double> st, stress, de6, dep;   // the replay by groups: state, new stress, strain increment
+    DVec<int> lists;                     // its list heads, 8 per increment run
 };
 
 struct fas_handle {
@@ -1115,7 +1117,15 @@ int create_impl(fas_handle *h, const fas_mesh_desc *Md, const fas_matl_desc *T, 
             const int ns = h->M.ns[std::abs(h->h_gp_iel[g]) - 1];
             ++h->cp_class[ns <= 12 ? 0 : ns <= 32 ? 1 : 2].n;
         }
-        for (int c = 0; c < 3; ++c) h->cp_class[c].ns = bound[c];
+        int by_gp[3] = {0, 0, 0};    // the replays' items are the GPs
+        for (int g = 0; g < h->ngps; ++g) {
+            const int ns = h->M.ns[std::abs(h->h_gp_iel[g]) - 1];
+            ++by_gp[ns <= 12 ? 0 : ns <= 32 ? 1 : 2];
+        }
+        for (int c = 0; c < 3; ++c) {
+            h->cp_class[c].ns = bound[c];
+            h->cp_class[c].n = std::max(h->cp_class[c].n, by_gp[c]);
+        }
     }
     h->ns_tmpl = h->maxns <= 12 ? 12 : (h->maxns <= 32 ? 32 : 60);
     // tables in shared memory (FAS_SMEM_TABLES builds) when they fit the
@@ -1248,6 +1258,7 @@ int down_field(fas_handle *h, void *dst, int rb, int ld, int nk, int n, const do
 }
 
 int prepare_solve(fas_handle *h);
+bool group_pass(const fas_handle *h);
 int ensure_group(fas_handle *h);
 
 int upload_impl(fas_handle *h, const fas_state_desc *S)
@@ -1292,7 +1303,7 @@ int upload_impl(fas_handle *h, const fas_state_desc *S)
         if (!rc) rc = prepare_solve(h);
         if (rc) return rc;
     }
-    if (!h->have_state && (rc = ensure_group(h))) return rc;
+    if (!h->have_state && group_pass(h) && (rc = ensure_group(h))) return rc;
     CK(cudaStreamSynchronize(h->stream));
     h->have_state = true;
     return 0;
@@ -1396,7 +1407,7 @@ bool group_pass(const fas_handle *h)
 // kernels.
 int ensure_group(fas_handle *h)
 {
-    if (!group_pass(h)) return 0;
+    if (!h->cp_group) return 0;
     cudaError_t e = cudaSuccess;
     if (!h->cp_w.p) e = h->cp_w.alloc(CPW * (size_t)h->ngps);
     if (e == cudaSuccess && !h->cp_queue.p) e = h->cp_queue.alloc(8);
@@ -1426,7 +1437,24 @@ CpWork group_work(fas_handle *h)
     w.off_s = 3 * h->nn;
     w.gp_of = h->point_mode ? nullptr : h->gp_item.p;
     w.gp_iel = h->gp_iel.p;
+    w.stress = nullptr;
     return w;
+}
+
+// The iterations of list k, on as many CTAs as reside at once.
+int launch_cp(fas_handle *h, int k, const DevGp &G, const CpWork &W, double dt, int inc, int nit)
+{
+    auto &c = h->cp_class[k];
+    const auto kern = cp_kernel(c.ns);
+    if (c.grid == 0) {
+        int occ = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, CP_THREADS, 0));
+        c.grid = std::max(occ, 1) * h->nsm;
+    }
+    const unsigned blk = std::min<unsigned>(c.grid, nblocks((long long)c.n * cp_lanes(c.ns), CP_THREADS));
+    kern<<<blk, CP_THREADS, 0, h->stream>>>(h->M, h->C, G, W, k, dt, inc, nit, h->ekey.p);
+    LAUNCHED(h);
+    return 0;
 }
 
 // DSTRSS of every GP by the group pass: kinematics and what a point does once,
@@ -1448,15 +1476,7 @@ int launch_group(fas_handle *h, double dt, int inc, int nit)
     for (int k = 0; k < 3; ++k) {
         auto &c = h->cp_class[k];
         if (c.n == 0) continue;
-        const auto kern = cp_kernel(c.ns);
-        if (c.grid == 0) {
-            int occ = 0;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, CP_THREADS, 0));
-            c.grid = std::max(occ, 1) * h->nsm;
-        }
-        const unsigned blk = std::min<unsigned>(c.grid, nblocks((long long)c.n * cp_lanes(c.ns), CP_THREADS));
-        kern<<<blk, CP_THREADS, 0, s>>>(h->M, h->C, h->gp(), W, k, dt, inc, nit, h->ekey.p);
-        LAUNCHED(h);
+        if (int rc = launch_cp(h, k, h->gp(), W, dt, inc, nit)) return rc;
         cp_tangent_kernel()<<<nblocks(c.n, 128), 128, 0, s>>>(h->gp(), W, k);
         LAUNCHED(h);
     }
@@ -1469,7 +1489,8 @@ int launch_elem(fas_handle *h, int inc, int nit)
     const int ns = h->ns_tmpl;
     const double dt = h->h_tiem[inc - 1];
     int *queue = nullptr, bs = 128;
-    if (int rc = ensure_group(h)) return rc;
+    if (group_pass(h))
+        if (int rc = ensure_group(h)) return rc;
     const bool group = group_pass(h);
     if (group) {
         if (int rc = launch_group(h, dt, inc, nit)) return rc;
@@ -2329,7 +2350,8 @@ int ensure_inc_graph(fas_handle *h, int inc, cudaGraphExec_t *out)
     // the solve's and the work order's buffers are sized outside the capture
     if (flow_on(h, fp32))
         if (int rc = fp32 ? ensure_flow<float>(h) : ensure_flow<double>(h)) return rc;
-    if (int rc = ensure_group(h)) return rc;
+    if (group_pass(h))
+        if (int rc = ensure_group(h)) return rc;
     if (group_pass(h)) {
     } else if (h->nn != 8)
         work_order(h, h->npg * h->nlmnt, h->gp_item.p);
@@ -2576,6 +2598,104 @@ void launch_replay_adj(fas_handle *h, const ReplayDev &H, const DevGp &G, int rs
                                                                   h->rp.gsv.p, h->rp.gp.p, h->ekey.p);
 }
 
+// The replay by groups of lanes (fas_replay_group.cuh): its buffers, or
+// `ready` false where the materials or the memory left call for a thread per GP.
+// The rule is the group pass's: 4,096 points and 20 increments 9.6 against 147 ms,
+// one increment of as
+// many points 0.75 against 3.6.
+int replay_group_prepare(fas_handle *h, const fas_replay_desc *d, DevGp &G, bool &ready)
+{
+    ready = false;
+    if (h->cp_group)
+        if (int rc = ensure_group(h)) return rc;
+    if (!h->cp_group) return 0;
+    ReplayBufs &B = h->rp;
+    const size_t ng = h->ngps;
+    cudaError_t e = cudaSuccess;
+    for (auto *v : {&B.st, &B.stress, &B.de6})
+        if (e == cudaSuccess) e = ensure(*v, 6 * ng);
+    if (e == cudaSuccess) e = ensure(B.dep, ng);
+    if (e == cudaSuccess) e = ensure(B.lists, 16 * (size_t)d->ninc);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return 0;
+    }
+    CKA(e);
+    CK(cudaMemcpyAsync(B.st.p, h->st.p, 6 * ng * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemsetAsync(B.lists.p, 0, 16 * (size_t)d->ninc * sizeof(int), h->stream));
+    CK(cudaMemsetAsync(B.cp_iters.p, 0, ng * sizeof(int), h->stream));
+    G.st = B.st.p;
+    G.de = B.de6.p;
+    G.dep = B.dep.p;
+    ready = true;
+    return 0;
+}
+
+// Increments n0 .. n1 - 1 forwards, from checkpoint rows `load` (null: from the
+// state in G).  `record`: the first recorded increment (n1: none), whose rows
+// start the record buffer; `chk`: whether to write checkpoints.  `run` counts
+// the increments run so far, each with list heads of its own.
+int replay_group_forward(fas_handle *h, const fas_replay_desc *d, const ReplayDev &H, DevGp G, int rs, int n0, int n1, int record,
+                         const double *load, bool chk, int &run)
+{
+    ReplayBufs &B = h->rp;
+    const size_t ng = h->ngps;
+    CpWork W = group_work(h);
+    W.rec = nullptr;
+    W.gp_of = nullptr;
+    W.stress = B.stress.p;
+    double *const srate = G.srate;
+    auto rows_of = [&](int n) { return n >= record && n < n1 ? B.rec.p + (size_t)(n - record) * rs * ng : nullptr; };
+    for (int n = n0; n <= n1; ++n) {
+        ReplayRows rows;
+        rows.commit = n > n0 ? rows_of(n - 1) : nullptr;
+        rows.next = rows_of(n);
+        rows.chk = chk && n < n1 && n % H.chk == 0 ? B.chk.p + (size_t)(n / H.chk) * H.zs * ng : nullptr;
+        rows.load = n == n0 ? load : nullptr;
+        rows.flag = H.zs + 6 + h->ns_tmpl;
+        W.count = B.lists.p + 8 * run;
+        W.head = W.count + 4;
+        replay_step_kernel()<<<nblocks(ng, 64), 64, 0, h->stream>>>(h->M, G, W, H, rows, n, n > n0, n < n1, h->ekey.p);
+        LAUNCHED(h);
+        if (n == n1) break;
+        // the slip rates go straight to the record
+        G.srate = rows.next ? rows.next + (size_t)(H.zs + 6) * ng : srate;
+        for (int k = 0; k < 3; ++k)
+            if (h->cp_class[k].n > 0)
+                if (int rc = launch_cp(h, k, G, W, d->dt[n], n + 1, 1)) return rc;
+        ++run;
+    }
+    return 0;
+}
+
+// The objective and, with `grad`, its adjoints: the whole history forwards,
+// recording the last segment, then segment by segment backwards.
+int replay_group(fas_handle *h, const fas_replay_desc *d, const ReplayDev &H, const DevGp &G, int rs, bool grad)
+{
+    ReplayBufs &B = h->rp;
+    const size_t ng = h->ngps;
+    const int nlast = (H.ninc - 1) / H.chk * H.chk;
+    int run = 0;
+    if (int rc = replay_group_forward(h, d, H, G, rs, 0, H.ninc, grad ? nlast : H.ninc, nullptr, grad, run)) return rc;
+    replay_seed_kernel()<<<nblocks(ng, 64), 64, 0, h->stream>>>(h->M, G, h->gp_iel.p, H, B.jg.p, B.eq.p, grad ? B.gst.p : nullptr,
+                                                                grad ? B.gsv.p : nullptr, grad ? B.gp.p : nullptr);
+    LAUNCHED(h);
+    if (!grad) return 0;
+    // the recomputed increments start from the same twin state as the first run
+    CK(cudaMemcpyAsync(B.twinsys.p, h->twinsys.p, ng * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+    const long long threads = (long long)ng * cp_lanes(h->ns_tmpl);
+    for (int n0 = nlast; n0 >= 0; n0 -= H.chk) {
+        const int n1 = std::min(H.ninc, n0 + H.chk);
+        if (n0 < nlast)
+            if (int rc = replay_group_forward(h, d, H, G, rs, n0, n1, n0, B.chk.p + (size_t)(n0 / H.chk) * H.zs * ng, false, run))
+                return rc;
+        replay_rev_kernel(h->ns_tmpl)<<<nblocks(threads, 64), 64, 0, h->stream>>>(
+            h->M, G, h->gp_iel.p, H, B.rec.p, rs, H.zs + 6 + h->ns_tmpl, n0, n1, B.gst.p, B.gsv.p, B.gp.p, h->ekey.p);
+        LAUNCHED(h);
+    }
+    return 0;
+}
+
 // Waits for the replay kernels; the objective summed over the GPs in GP order.
 int replay_finish(fas_handle *h, double *J)
 {
@@ -2793,7 +2913,8 @@ int32_t fas_gpu_constitutive(fas_handle *h, int32_t inc, int32_t nit)
     CK(cudaMemsetAsync(h->ekey.p, 0xFF, sizeof(unsigned long long), s));
     Span sp(h, &h->P.ms_constitutive);
     const double dt = h->h_tiem[inc - 1];
-    if (int rc = ensure_group(h)) return rc;
+    if (group_pass(h))
+        if (int rc = ensure_group(h)) return rc;
     const bool group = group_pass(h) && h->point_mode;
     if (group) {
         if (int rc = launch_group(h, dt, inc, nit)) return rc;
@@ -2876,9 +2997,16 @@ int32_t fas_gpu_adjoint_forward(fas_handle *h, const fas_replay_desc *d, double 
     DevGp G;
     int rs = 0;
     int rc = replay_prepare(h, d, false, H, G, rs);
+    bool group = false;
+    if (!rc) rc = replay_group_prepare(h, d, G, group);
     if (rc) return rc;
-    launch_replay_fwd(h, H, G, 0);
-    LAUNCHED(h);
+    if (group) {
+        rc = replay_group(h, d, H, G, rs, false);
+        if (rc) return rc;
+    } else {
+        launch_replay_fwd(h, H, G, 0);
+        LAUNCHED(h);
+    }
     rc = replay_finish(h, J);
     if (rc) return rc;
     if (eq) CK(cudaMemcpy(eq, h->rp.eq.p, h->ngps * sizeof(double), cudaMemcpyDeviceToHost));
@@ -2892,14 +3020,21 @@ int32_t fas_gpu_adjoint_grad(fas_handle *h, const fas_replay_desc *d, double *J,
     DevGp G;
     int rs = 0;
     int rc = replay_prepare(h, d, true, H, G, rs);
+    bool group = false;
+    if (!rc) rc = replay_group_prepare(h, d, G, group);
     if (rc) return rc;
     const size_t ng = h->ngps;
-    launch_replay_fwd(h, H, G, rs);
-    LAUNCHED(h);
-    // the reverse sweep starts from the same twin state as the forward one
-    CK(cudaMemcpyAsync(h->rp.twinsys.p, h->twinsys.p, ng * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
-    launch_replay_adj(h, H, G, rs);
-    LAUNCHED(h);
+    if (group) {
+        rc = replay_group(h, d, H, G, rs, true);
+        if (rc) return rc;
+    } else {
+        launch_replay_fwd(h, H, G, rs);
+        LAUNCHED(h);
+        // the reverse sweep starts from the same twin state as the forward one
+        CK(cudaMemcpyAsync(h->rp.twinsys.p, h->twinsys.p, ng * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+        launch_replay_adj(h, H, G, rs);
+        LAUNCHED(h);
+    }
     rc = replay_finish(h, J);
     if (rc) return rc;
     const int nsv = 3 + h->maxns;

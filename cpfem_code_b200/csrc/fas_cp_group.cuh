@@ -38,133 +38,9 @@
 // the general path's to rounding (fas_device.cuh: dstrss).
 #pragma once
 
-#include <type_traits>
-
-#include "fas_device.cuh"
-#include "fas_cp_types.h"
-#include "fas_layout.cuh"
+#include "fas_cp_math.cuh"
 
 namespace fasdev {
-
-template <int NS> struct GpShape {
-    static constexpr int L = NS <= 12 ? 4 : NS <= 32 ? 8 : 16;   // lanes per point
-    static constexpr int P = (NS + L - 1) / L;                   // systems per lane
-};
-
-constexpr unsigned ALL = 0xffffffffu;
-
-template <int L> __device__ __forceinline__ double gsum(double v)
-{
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(ALL, v, o);
-    return v;
-}
-template <int L> __device__ __forceinline__ double gmax(double v)
-{
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) v = fmax(v, __shfl_xor_sync(ALL, v, o));
-    return v;
-}
-template <int L> __device__ __forceinline__ int gmin(int v)
-{
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) v = min(v, __shfl_xor_sync(ALL, v, o));
-    return v;
-}
-template <int L> __device__ __forceinline__ int gisum(int v)
-{
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) v += __shfl_xor_sync(ALL, v, o);
-    return v;
-}
-
-// ELASTC (src/fasolt/ela-plas.f90:12-86) from CTMATRX's a, upper triangle
-// S[utri(I, J)]; the products of two direction cosines are formed once.
-__device__ __forceinline__ void elastc_upper(const double *e, const double a0[3][3], double S[21])
-{
-    const int pi[6] = {0, 1, 2, 1, 2, 0}, pj[6] = {0, 1, 2, 2, 0, 1};
-    double ev[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) ev[k] = __ldg(e + k);
-    double d[6][3], x[6][6];   // a_ip a_jp, and a_ip a_jq for the pairs (p, q) = 12, 21, 20, 02, 01, 10
-#pragma unroll
-    for (int I = 0; I < 6; ++I) {
-        const int i = pi[I], j = pj[I];
-#pragma unroll
-        for (int p = 0; p < 3; ++p) d[I][p] = a0[p][i] * a0[p][j];
-        x[I][0] = a0[1][i] * a0[2][j];
-        x[I][1] = a0[2][i] * a0[1][j];
-        x[I][2] = a0[2][i] * a0[0][j];
-        x[I][3] = a0[0][i] * a0[2][j];
-        x[I][4] = a0[0][i] * a0[1][j];
-        x[I][5] = a0[1][i] * a0[0][j];
-    }
-#pragma unroll
-    for (int I = 0; I < 6; ++I)
-#pragma unroll
-        for (int J = I; J < 6; ++J) {
-            double v = d[I][0] * d[J][0] * ev[0] + d[I][1] * d[J][1] * ev[1] + d[I][2] * d[J][2] * ev[2];
-            v += (d[I][1] * d[J][2] + d[I][2] * d[J][1]) * ev[3] + (d[I][2] * d[J][0] + d[I][0] * d[J][2]) * ev[4] +
-                 (d[I][0] * d[J][1] + d[I][1] * d[J][0]) * ev[5];
-            v += 0.5 * ((x[I][0] * x[J][0] + x[I][1] * x[J][1]) * ev[6] + (x[I][2] * x[J][2] + x[I][3] * x[J][3]) * ev[7] +
-                        (x[I][4] * x[J][4] + x[I][5] * x[J][5]) * ev[8]);
-            S[utri(I, J)] = I < 3 ? v : 2.0 * v;
-        }
-}
-
-// 6 x 6 elimination without pivoting (FACTOR), unrolled, with the reciprocal
-// pivots kept in place of the pivots; 1 for a zero pivot.
-__device__ __forceinline__ int lu6(double A[36])
-{
-    int bad = 0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        if (A[7 * k] == 0.0) bad = 1;
-        A[7 * k] = 1.0 / A[7 * k];
-#pragma unroll
-        for (int i = k + 1; i < 6; ++i) {
-            const double l = A[6 * i + k] * A[7 * k];
-            A[6 * i + k] = l;
-#pragma unroll
-            for (int j = k + 1; j < 6; ++j) A[6 * i + j] -= l * A[6 * k + j];
-        }
-    }
-    return bad;
-}
-// Solution of A x = y; `first` is the index of y's first nonzero entry.
-template <int FIRST> __device__ __forceinline__ void lu6_solve(const double A[36], double x[6])
-{
-#pragma unroll
-    for (int i = FIRST + 1; i < 6; ++i)
-#pragma unroll
-        for (int j = FIRST; j < i; ++j) x[i] -= A[6 * i + j] * x[j];
-#pragma unroll
-    for (int i = 5; i >= 0; --i) {
-#pragma unroll
-        for (int j = i + 1; j < 6; ++j) x[i] -= A[6 * i + j] * x[j];
-        x[i] *= A[7 * i];
-    }
-}
-// The symmetrised inverse (A^-1 + A^-T) / 2, upper triangle.
-__device__ __forceinline__ void lu6_inverse(const double A[36], double inv[21])
-{
-#pragma unroll
-    for (int k = 0; k < 21; ++k) inv[k] = 0.0;
-    auto column = [&](auto first) {
-        constexpr int c = decltype(first)::value;
-        double x[6] = {0, 0, 0, 0, 0, 0};
-        x[c] = 1.0;
-        lu6_solve<c>(A, x);
-#pragma unroll
-        for (int i = 0; i < 6; ++i) inv[i < c ? utri(i, c) : utri(c, i)] += i == c ? x[i] : 0.5 * x[i];
-    };
-    column(std::integral_constant<int, 0>{});
-    column(std::integral_constant<int, 1>{});
-    column(std::integral_constant<int, 2>{});
-    column(std::integral_constant<int, 3>{});
-    column(std::integral_constant<int, 4>{});
-    column(std::integral_constant<int, 5>{});
-}
 
 // ------------------------------------------------------------ before the iterations
 // What a point does once, by one thread: compliance and rotated stress; the
@@ -185,24 +61,7 @@ __device__ __forceinline__ void cp_prep(const DevMat &M, const DevGp &G, const C
     for (int k = 0; k < 6; ++k) s[k] = t[k] + G.ds[k * ng + g];
     const double einit = fj2vom(false, de);
     if (iel > 0 && fj2vom(true, s) > 0.0 && einit > 0.0) {
-#pragma unroll
-        for (int k = 0; k < 21; ++k) W.w[(size_t)k * ng + g] = S[k];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            W.w[(size_t)(CPW_T + k) * ng + g] = t[k];
-            W.w[(size_t)(CPW_S + k) * ng + g] = s[k];
-        }
-#pragma unroll
-        for (int k = 0; k < 9; ++k) W.w[(size_t)(CPW_A + k) * ng + g] = a[k / 3][k % 3];
-        W.w[(size_t)CPW_CAP * ng + g] = 6.0 * einit;
-        const int c = ns <= 12 ? 0 : ns <= 32 ? 1 : 2;
-        // one atomic per class and warp; the list keeps the items' order in the warp
-        const unsigned peers = __match_any_sync(__activemask(), c);
-        const int me = threadIdx.x & 31, lead = __ffs(peers) - 1;
-        int base = 0;
-        if (me == lead) base = atomicAdd(W.count + c, __popc(peers));
-        base = __shfl_sync(peers, base, lead);
-        W.list[c][base + __popc(peers & ((1u << me) - 1u))] = item;
+        cp_enlist(W, ng, item, g, ns, S, t, s, a, 6.0 * einit);
         return;
     }
     double A[36], inv[21], tn[6];
@@ -687,7 +546,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
 #pragma unroll
             for (int k = 0; k < 6; ++k) s[k] = s[k] + scale * err[k];
             fin = run && (rc != 0 || !(iter < C.maxit && em > C.toler));
-            if (fin && !rc) {
+            if (fin && !rc && !W.stress) {
 #pragma unroll
                 for (int k = 0; k < 36; ++k)
                     if (k % L == lane) W.w[(size_t)k * ng + g] = A[k];
@@ -711,7 +570,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
         for (int k = 0; k < 3; ++k) rtn[k] = gsum<L>(rtn[k]);
         if (fin) {
             if (lane == 0) {
-                G.cp_iters[g] = iter;
+                G.cp_iters[g] = rc && W.stress ? -1 : iter;
                 G.ops[g] = ops;
                 G.twinsys[g] = twinsys;
                 G.erepmd[g] = rc ? 0.0 : em;
@@ -726,7 +585,8 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
 #pragma unroll
                 for (int k = 0; k < 6; ++k)
                     if (k % L == lane) {
-                        G.ds[k * ng + g] = s[k] - G.st[k * ng + g];
+                        if (W.stress) W.stress[(size_t)k * ng + g] = s[k];
+                        else G.ds[k * ng + g] = s[k] - G.st[k * ng + g];
                         if (R) R[k] = s[k];
                     }
 #pragma unroll
@@ -758,21 +618,16 @@ __global__ void __launch_bounds__(128) k_cp_tangent(DevGp G, CpWork W, int cls)
     if (item < 0) return;
     const int g = W.gp_of ? W.gp_of[item] : item, ng = G.ngps;
     {
-        double a[3][3], aug[3], rx[3], sk[3], r[3];
+        double a[3][3], aug[3], dph[3], sk[3], r[3];
         ctmatrx(G.sv[g] + G.dsv[g], G.sv[ng + g] + G.dsv[ng + g], G.sv[2 * ng + g] + G.dsv[2 * ng + g], a, aug);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             sk[k] = W.w[(size_t)(CPW_SPIN + k) * ng + g];
             r[k] = G.dr[k * ng + g];
         }
-        // a (a^T skew - r) = skew - a r
+        echrot(a, aug, sk, r, dph);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) rx[k] = sk[k] - (a[k][0] * r[0] + a[k][1] * r[1] + a[k][2] * r[2]);
-        const double rz = a[0][2] * sk[0] + a[1][2] * sk[1] + a[2][2] * sk[2] - r[2];
-        const double dp1 = fabs(aug[2]) < 1.e-5 ? rz : (aug[0] * rx[0] + aug[1] * rx[1]) / aug[2];
-        G.dsv[g] = dp1;
-        G.dsv[ng + g] = aug[1] * rx[0] - aug[0] * rx[1];
-        G.dsv[2 * ng + g] = rx[2] - dp1 * a[2][2];
+        for (int k = 0; k < 3; ++k) G.dsv[k * ng + g] = dph[k];
     }
     double A[36], inv[21];
 #pragma unroll

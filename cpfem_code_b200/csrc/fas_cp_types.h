@@ -20,6 +20,8 @@ struct CpWork {
     int reclen, off_s;
     const int *gp_of;            // Gauss point of an item (null: the item itself)
     const int *gp_iel;
+    double *stress;              // replays: new stress [6][ngps] in place of G.ds; no tangent, and
+                                 // cp_iters -1 for a point that fails
 };
 
 }  // namespace fasdev

@@ -29,6 +29,11 @@ using ReplayFwdFn = void (*)(DevMat, DevCtrl, DevGp, const int *, const double *
 using ReplayAdjFn = void (*)(DevMat, DevCtrl, DevGp, const int *, ReplayDev, const double *, double *, int, double *,
                              double *, double *, double *, unsigned long long *);
 
+using ReplayStepFn = void (*)(DevMat, DevGp, CpWork, ReplayDev, ReplayRows, int, bool, bool, unsigned long long *);
+using ReplaySeedFn = void (*)(DevMat, DevGp, const int *, ReplayDev, double *, double *, double *, double *, double *);
+using ReplayRevFn = void (*)(DevMat, DevGp, const int *, ReplayDev, const double *, int, int, int, int, double *, double *,
+                             double *, unsigned long long *);
+
 // ns: the compile-time bound on slip systems (12, 32 or 60; 12 or 32 for
 // the warp and replay kernels); nn: nodes of a quadratic element (10, 15, 20)
 ElemFn elem_kernel(int ns);
@@ -44,5 +49,8 @@ Prep8Fn prep8_kernel();
 PrepqFn prepq_kernel(int nn);
 ReplayFwdFn replay_fwd_kernel(int ns);
 ReplayAdjFn replay_adj_kernel(int ns);
+ReplayStepFn replay_step_kernel();
+ReplaySeedFn replay_seed_kernel();
+ReplayRevFn replay_rev_kernel(int ns);
 
 }  // namespace fasdev

@@ -1,0 +1,584 @@
+// fas_replay_group.cuh -- the replay and its adjoint (fas_adjoint.cuh has the
+// definitions) for materials that the group pass serves.
+//
+// What bounded the adjoint.  One thread per Gauss point ran DSTRSS and, for an
+// increment backwards, one dual pass of the local system per input (12 to 40 of
+// them) and an elimination, all in local memory: 4,096 points and 20 increments
+// took 147 ms.  Here
+//   * an increment forwards is k_cp with lanes sharing a point; k_replay_step
+//     commits the increment before and prepares the next, one thread per point;
+//   * an increment backwards is written out.  lambda of an active system is an
+//     affine function of lambda_s (6), of C = sum_i c_i and of
+//     W = sum_j h'_j |g_j| H_j, where c_i = ybar_i + lambda_i / s1_i is what
+//     weighs s1_i, H_j = q C + (d_j - q) c_j and h' the derivative of gradh by
+//     the sum of slips (A6).  That leaves one symmetric positive 6 x 6 system
+//     with two more unknowns, whose entries are sums over the lanes' systems;
+//   * the derivatives by the Euler angles go through the direction cosines a:
+//     abar collects what the slip systems, ELASTC and ECHROT pass back.
+// The matrices are those of the dual passes, in another order of summation.
+// 4,096 points and 20 increments now take 9.6 ms with segments of five: 35
+// increments forwards at 0.25 ms (k_cp 0.23), four segments backwards at 0.11 ms.
+// Both are one dependent chain per point with a warp or two per scheduler.  The
+// gradient's error against the same in more digits went from 8.9e-13 to 5.8e-13.
+#pragma once
+
+#include "fas_adjoint_types.cuh"
+#include "fas_cp_math.cuh"
+
+namespace fasdev {
+
+// F = sum_ij l_i S_ij u_j with ELASTC's S (elastc_upper), S = f_I^T E f_J times
+// 2 where both I, J >= 3; abar[p][i] += scale dF / da[p][i] if asked for.
+template <bool GRAD>
+__device__ __forceinline__ double compliance_form(const double *e9, const double a[3][3], const double l[6], const double u[6],
+                                                  double scale, double abar[3][3])
+{
+    const int pi[6] = {0, 1, 2, 1, 2, 0}, pj[6] = {0, 1, 2, 2, 0, 1};
+    double e[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) e[k] = __ldg(e9 + k);
+    double L[2][9], U[2][9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) L[0][k] = L[1][k] = U[0][k] = U[1][k] = 0.0;
+#pragma unroll
+    for (int I = 0; I < 6; ++I) {
+        const int i = pi[I], j = pj[I], b = I < 3 ? 0 : 1;
+        const double f[9] = {a[0][i] * a[0][j], a[1][i] * a[1][j], a[2][i] * a[2][j], a[1][i] * a[2][j], a[2][i] * a[1][j],
+                             a[2][i] * a[0][j], a[0][i] * a[2][j], a[0][i] * a[1][j], a[1][i] * a[0][j]};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            L[b][k] += l[I] * f[k];
+            U[b][k] += u[I] * f[k];
+        }
+    }
+    auto times_e = [&](const double v[9], double m, const double w[9], double out[9]) {   // E (v + m w)
+        double x[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) x[k] = v[k] + m * w[k];
+        out[0] = e[0] * x[0] + e[5] * x[1] + e[4] * x[2];
+        out[1] = e[5] * x[0] + e[1] * x[1] + e[3] * x[2];
+        out[2] = e[4] * x[0] + e[3] * x[1] + e[2] * x[2];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) out[3 + k] = 0.5 * e[6 + k / 2] * x[3 + k];
+    };
+    double EU[2][9], F = 0.0;
+    times_e(U[0], 1.0, U[1], EU[0]);
+    times_e(U[0], 2.0, U[1], EU[1]);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) F += L[0][k] * EU[0][k] + L[1][k] * EU[1][k];
+    if (GRAD) {
+        double EL[2][9];
+        times_e(L[0], 1.0, L[1], EL[0]);
+        times_e(L[0], 2.0, L[1], EL[1]);
+#pragma unroll
+        for (int I = 0; I < 6; ++I) {
+            const int i = pi[I], j = pj[I], b = I < 3 ? 0 : 1;
+            double w[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) w[k] = scale * (l[I] * EU[b][k] + u[I] * EL[b][k]);
+            const int p1[9] = {0, 1, 2, 1, 2, 2, 0, 0, 1}, p2[9] = {0, 1, 2, 2, 1, 0, 2, 1, 0};   // f_k = a[p1][i] a[p2][j]
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                abar[p1[k]][i] += w[k] * a[p2[k]][j];
+                abar[p2[k]][j] += w[k] * a[p1[k]][i];
+            }
+        }
+    }
+    return F;
+}
+
+// S u with S's upper triangle
+__device__ __forceinline__ void sym6(const double S[21], const double u[6], double y[6])
+{
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        double acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) acc += S[i <= j ? utri(i, j) : utri(j, i)] * u[j];
+        y[i] = acc;
+    }
+}
+
+// Adjoint of CTMATRX: what abar and the adjoints of aug = (sin, cos of the
+// third, sin of the second angle) pass to the Euler angles.
+__device__ __forceinline__ void angles_bar(const double ph[3], const double a[3][3], const double abar[3][3],
+                                           const double augbar[3], double phbar[3])
+{
+    double s1, c1, s, c, s2, c2;
+    sincos(ph[0], &s1, &c1);
+    sincos(ph[1], &s, &c);
+    sincos(ph[2], &s2, &c2);
+    phbar[0] += abar[0][1] * a[0][0] - abar[0][0] * a[0][1] + abar[1][1] * a[1][0] - abar[1][0] * a[1][1] +
+                abar[2][1] * a[2][0] - abar[2][0] * a[2][1];
+    phbar[1] += s2 * (abar[0][0] * a[2][0] + abar[0][1] * a[2][1]) + c2 * (abar[1][0] * a[2][0] + abar[1][1] * a[2][1]) +
+                c * (s1 * abar[2][0] - c1 * abar[2][1] + s2 * abar[0][2] + c2 * abar[1][2]) - s * abar[2][2] + c * augbar[2];
+    phbar[2] += abar[0][0] * a[1][0] - abar[1][0] * a[0][0] + abar[0][1] * a[1][1] - abar[1][1] * a[0][1] +
+                abar[0][2] * a[1][2] - abar[1][2] * a[0][2] + c2 * augbar[0] - s2 * augbar[1];
+}
+
+// ------------------------------------------------------------ forwards
+// Commits increment n - 1 (if it ran) and prepares increment n (if n < last):
+// its input state to the record and the checkpoint, the elastic predictor, the
+// points that take CPSTRS to their lists.  G.st and G.sv hold the state; a point
+// that has failed (cp_iters < 0) stays as it is.
+__global__ void __launch_bounds__(64) k_replay_step(DevMat M, DevGp G, CpWork W, ReplayDev H, ReplayRows rows, int n, bool commit,
+                                                    bool next, unsigned long long *errkey)
+{
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int ng = G.ngps;
+    if (g >= ng || G.cp_iters[g] < 0) return;
+    const int iel = W.gp_iel[g], mc = (iel < 0 ? -iel : iel) - 1, ns = M.ns[mc];
+    double st[6], ph[3];
+    if (commit) {
+        const bool plastic = G.cp_iters[g] > 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) st[k] = W.stress[(size_t)k * ng + g];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ph[k] = G.sv[(size_t)k * ng + g];
+        if (plastic) {
+            double a[3][3], aug[3], sk[3], r[3], dph[3];
+            ctmatrx(ph[0], ph[1], ph[2], a, aug);
+            const double *pr = H.dr + ((size_t)(n - 1) * ng + g) * 3;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                sk[k] = W.w[(size_t)(CPW_SPIN + k) * ng + g];
+                r[k] = pr[k];
+            }
+            echrot(a, aug, sk, r, dph);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ph[k] = ph[k] + dph[k];
+                G.sv[(size_t)k * ng + g] = ph[k];
+            }
+            for (int i = 3; i < 3 + ns; ++i)
+                G.sv[(size_t)i * ng + g] = G.sv[(size_t)i * ng + g] + G.dsv[(size_t)i * ng + g];
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) G.st[(size_t)k * ng + g] = st[k];
+        if (rows.commit) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) rows.commit[(size_t)(H.zs + k) * ng + g] = st[k];
+            if (!plastic)
+                for (int i = 0; i < ns; ++i) rows.commit[(size_t)(H.zs + 6 + i) * ng + g] = 0.0;
+            rows.commit[(size_t)rows.flag * ng + g] = plastic ? 1.0 : 0.0;
+        }
+    } else {
+        const double *c = rows.load;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            st[k] = c ? c[(size_t)k * ng + g] : G.st[(size_t)k * ng + g];
+            if (c) G.st[(size_t)k * ng + g] = st[k];
+        }
+        if (c)
+            for (int i = 0; i < 3 + ns; ++i) G.sv[(size_t)i * ng + g] = c[(size_t)(6 + i) * ng + g];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ph[k] = G.sv[(size_t)k * ng + g];
+    }
+    if (!next) return;
+    auto state_to = [&](double *p) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) p[(size_t)k * ng + g] = st[k];
+        for (int i = 0; i < 3 + ns; ++i) p[(size_t)(6 + i) * ng + g] = G.sv[(size_t)i * ng + g];
+    };
+    if (rows.chk) state_to(rows.chk);
+    if (rows.next) state_to(rows.next);
+    double de[6], r[3], t[6], s[6], a[3][3], aug[3], S[21], A[36], pred[6];
+    const double *pe = H.de + ((size_t)n * ng + g) * 6, *pr = H.dr + ((size_t)n * ng + g) * 3;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        pred[k] = de[k] = pe[k];
+        G.de[(size_t)k * ng + g] = de[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r[k] = pr[k];
+    ctmatrx(ph[0], ph[1], ph[2], a, aug);
+    elastc_upper(M.e + 9 * mc, a, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int j = 0; j < 6; ++j) A[6 * i + j] = S[i <= j ? utri(i, j) : utri(j, i)];
+    if (lu6(A)) {
+        atomicMin(errkey, ((unsigned long long)g << 16) | 910ull);
+        G.cp_iters[g] = -1;
+        return;
+    }
+    lu6_solve<0>(A, pred);
+    tens_rot(r, st, t);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) s[k] = t[k] + pred[k];
+    const double einit = fj2vom(false, de);
+    if (iel > 0 && fj2vom(true, s) > 0.0 && einit > 0.0) {
+        cp_enlist(W, ng, g, g, ns, S, t, s, a, 6.0 * einit);
+        return;
+    }
+    G.cp_iters[g] = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) W.stress[(size_t)k * ng + g] = pred[k];
+}
+
+// The objective's share of each GP from the final state, and, with g_st, its
+// adjoints on that state.
+__global__ void __launch_bounds__(64) k_replay_seed(DevMat M, DevGp G, const int *gp_iel, ReplayDev H, double *Jg, double *eq,
+                                                    double *g_st, double *g_sv, double *g_p)
+{
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int ng = G.ngps;
+    if (g >= ng || G.cp_iters[g] < 0) return;
+    const int iel = gp_iel[g], mc = (iel < 0 ? -iel : iel) - 1, ns = M.ns[mc];
+    const double *q = H.q;
+    const double qq[6] = {q[0] * q[0], q[1] * q[1], q[2] * q[2], q[1] * q[2], q[2] * q[0], q[0] * q[1]};
+    double st[6], ph[3], a[3][3], aug[3], ab[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) st[k] = G.st[(size_t)k * ng + g];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) ph[k] = G.sv[(size_t)k * ng + g];
+    ctmatrx(ph[0], ph[1], ph[2], a, aug);
+    const double e = compliance_form<true>(M.e + 9 * mc, a, qq, st, 1.0, ab);
+    const double w = H.w[g], y = H.y[g], f = w * (e - y);
+    Jg[g] = 0.5 * w * (e - y) * (e - y);
+    eq[g] = e;
+    if (!g_st) return;
+    double S[21], x[6], pb[3] = {0.0, 0.0, 0.0};
+    const double none[3] = {0.0, 0.0, 0.0};
+    elastc_upper(M.e + 9 * mc, a, S);
+    sym6(S, qq, x);
+    angles_bar(ph, a, ab, none, pb);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) g_st[(size_t)k * ng + g] = f * x[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) g_sv[(size_t)k * ng + g] = f * pb[k];
+    for (int i = 0; i < ns; ++i) g_sv[(size_t)(3 + i) * ng + g] = 0.0;
+#pragma unroll
+    for (int k = 0; k < ADJ_NP; ++k) g_p[(size_t)k * ng + g] = 0.0;
+}
+
+// ------------------------------------------------------------ backwards
+// x^y as PLASTC takes it (x >= 0) and its derivative by x
+__device__ __forceinline__ void pow01_d(double x, double y, double &p, double &dp)
+{
+    if (y == 0.0) {
+        p = 1.0;
+        dp = 0.0;
+    } else if (y == 1.0) {
+        p = x;
+        dp = 1.0;
+    } else if (!(x > 0.0)) {
+        p = dp = 0.0;
+    } else {
+        p = exp(y * log(x));
+        dp = p * y / x;
+    }
+}
+
+// Increments n1 - 1 down to n0 backwards; g_st, g_sv and g_p hold the adjoints
+// of the state after them and receive those of the state before them.
+// `rec` holds the records of n0 .. n1 - 1.
+template <int NS>
+__global__ void __launch_bounds__(64) k_replay_rev(DevMat M, DevGp G, const int *gp_iel, ReplayDev H, const double *rec, int rs,
+                                                   int flag, int n0, int n1, double *g_st, double *g_sv, double *g_p,
+                                                   unsigned long long *errkey)
+{
+    constexpr int L = GpShape<NS>::L, P = GpShape<NS>::P;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, lane = tid % L, ng = G.ngps;
+    bool run = tid / L < ng;
+    const int g = run ? tid / L : ng - 1;
+    run = run && G.cp_iters[g] >= 0;
+    const int iel = gp_iel[g], mc = (iel < 0 ? -iel : iel) - 1, ns = M.ns[mc];
+    const double *amp = M.ampar + (size_t)mc * M.tld * 6, *sm = M.sm + (size_t)mc * M.sld;
+    const double qh = M.hq[mc];
+    bool on[P];
+    double ys[6], yph[3], y0[P], pbar[ADJ_NP];
+#pragma unroll
+    for (int k = 0; k < ADJ_NP; ++k) pbar[k] = g_p[(size_t)k * ng + g];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) ys[k] = g_st[(size_t)k * ng + g];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) yph[k] = g_sv[(size_t)k * ng + g];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        on[j] = lane + L * j < ns;
+        y0[j] = on[j] ? g_sv[(size_t)(3 + lane + L * j) * ng + g] : 0.0;
+    }
+    for (int n = n1 - 1; n >= n0; --n) {
+        const double *R = rec + (size_t)(n - n0) * rs * ng + g;
+        const bool plastic = R[(size_t)flag * ng] != 0.0;
+        const double dt = H.dt[n];
+        double s[6], t[6], u[6], r[3], ph[3], a[3][3], aug[3];
+        {
+            double st[6];
+            const double *pr = H.dr + ((size_t)n * ng + g) * 3;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                st[k] = R[(size_t)k * ng];
+                s[k] = R[(size_t)(H.zs + k) * ng];
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                ph[k] = R[(size_t)(6 + k) * ng];
+                r[k] = pr[k];
+            }
+            tens_rot(r, st, t);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) u[k] = plastic ? s[k] - t[k] : s[k];
+        }
+        ctmatrx(ph[0], ph[1], ph[2], a, aug);
+        // the lane's systems
+        double d[P][3], nn[P][3], tau[P], ag[P], sg[P], s0[P], slip = 0.0;
+        bool act[P];
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const int ii = on[j] ? lane + L * j : 0;
+            const double *pa = M.ab + ((size_t)mc * M.tld + ii) * 3, *pn = M.an + ((size_t)mc * M.tld + ii) * 3;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                d[j][k] = a[0][k] * __ldg(pa) + a[1][k] * __ldg(pa + 1) + a[2][k] * __ldg(pa + 2);
+                nn[j][k] = a[0][k] * __ldg(pn) + a[1][k] * __ldg(pn + 1) + a[2][k] * __ldg(pn + 2);
+            }
+            s0[j] = R[(size_t)(9 + ii) * ng];
+            ag[j] = on[j] ? R[(size_t)(H.zs + 6 + ii) * ng] * dt : 0.0;
+            act[j] = plastic && ag[j] > 0.0;
+            if (!act[j]) ag[j] = 0.0;
+            tau[j] = d[j][0] * nn[j][0] * s[0] + d[j][1] * nn[j][1] * s[1] + d[j][2] * nn[j][2] * s[2] +
+                     (d[j][1] * nn[j][2] + d[j][2] * nn[j][1]) * s[3] + (d[j][2] * nn[j][0] + d[j][0] * nn[j][2]) * s[4] +
+                     (d[j][0] * nn[j][1] + d[j][1] * nn[j][0]) * s[5];
+            sg[j] = copysign(1.0, tau[j]);
+            slip += ag[j];
+        }
+        slip = gsum<L>(slip);
+        // PLASTC and its derivatives
+        double gh[P], dh0[P], dh5[P], pw[P], eta[P], s1[P], hsum = 0.0;
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const double *p = amp + 6 * (on[j] ? lane + L * j : 0);
+            const double A2 = __ldg(p + 1), A5 = __ldg(p + 4);
+            double rate, drate, dpw;
+            pow01_d(slip / dt, __ldg(p + 5), rate, drate);
+            const double sst = A5 * rate;
+            double arg = sst != 0.0 ? 1.0 - s0[j] / sst : 0.0;
+            const bool cut = sst == 0.0 || arg < 0.0;
+            if (arg < 0.0) arg = 0.0;
+            pow01_d(arg, __ldg(p + 3), pw[j], dpw);
+            gh[j] = __ldg(p + 2) + A2 * pw[j];
+            dh0[j] = cut ? 0.0 : -(A2 * dpw / sst);
+            const double dsst = cut ? 0.0 : A2 * dpw * s0[j] / (sst * sst);
+            dh5[j] = dsst * rate;
+            eta[j] = act[j] ? dsst * A5 * drate / dt * ag[j] : 0.0;
+            hsum += gh[j] * ag[j];
+        }
+        hsum = gsum<L>(hsum);
+        // ECHROT: rtn = sum g (d x n) / 2 - r, and what its outputs pass back
+        double rtn[3] = {0.0, 0.0, 0.0}, rxb[3], augb[3], dp1, rtb[3], e0[P];
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const double h = act[j] ? 0.5 * (sg[j] * ag[j]) : 0.0;
+            rtn[0] += h * (d[j][1] * nn[j][2] - d[j][2] * nn[j][1]);
+            rtn[1] += h * (d[j][2] * nn[j][0] - d[j][0] * nn[j][2]);
+            rtn[2] += h * (d[j][0] * nn[j][1] - d[j][1] * nn[j][0]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) rtn[k] = gsum<L>(rtn[k]) - r[k];
+        {
+            double rx[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) rx[k] = a[k][0] * rtn[0] + a[k][1] * rtn[1] + a[k][2] * rtn[2];
+            const bool pole = fabs(aug[2]) < 1.e-5;
+            dp1 = pole ? rtn[2] : (aug[0] * rx[0] + aug[1] * rx[1]) / aug[2];
+            const double db = yph[0] - a[2][2] * yph[2], dv = pole ? 0.0 : db / aug[2];
+            rxb[0] = aug[1] * yph[1] + aug[0] * dv;
+            rxb[1] = aug[1] * dv - aug[0] * yph[1];
+            rxb[2] = yph[2];
+            augb[0] = rx[0] * dv - rx[1] * yph[1];
+            augb[1] = rx[0] * yph[1] + rx[1] * dv;
+            augb[2] = -(dp1 * dv);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) rtb[k] = a[0][k] * rxb[0] + a[1][k] * rxb[1] + a[2][k] * rxb[2];
+            if (pole) rtb[2] += db;
+        }
+        // lambda_j = k0 - sg iD (b . lambda_s) - iD gh q C - iD W
+        double iD[P], k0[P], ls[6], C, Wv;
+        double S[21];
+        elastc_upper(M.e + 9 * mc, a, S);
+        {
+            double A[36], x0[6], x1[6], x2[6], rowC[6], rowW[6];
+            double cc = 0.0, cw = 0.0, c0 = 0.0, wc = 0.0, ww = 0.0, w0 = 0.0, es = 0.0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) x0[k] = x1[k] = x2[k] = rowC[k] = rowW[k] = 0.0;
+#pragma unroll
+            for (int k = 0; k < 36; ++k) A[k] = 0.0;
+#pragma unroll
+            for (int j = 0; j < P; ++j) {
+                const int ii = on[j] ? lane + L * j : 0;
+                const double am = __ldg(amp + 6 * ii), dq = __ldg(sm + ii * ns + ii) - qh;
+                s1[j] = s0[j] + qh * hsum + dq * (gh[j] * ag[j]);
+                e0[j] = 0.5 * (rtb[0] * (d[j][1] * nn[j][2] - d[j][2] * nn[j][1]) + rtb[1] * (d[j][2] * nn[j][0] - d[j][0] * nn[j][2]) +
+                               rtb[2] * (d[j][0] * nn[j][1] - d[j][1] * nn[j][0]));
+                iD[j] = act[j] ? 1.0 / (am / ag[j] + gh[j] * dq / s1[j]) : 0.0;
+                k0[j] = -iD[j] * (sg[j] * e0[j] + gh[j] * dq * y0[j]);
+                c0 += y0[j];
+                if (act[j]) {
+                    const double b[6] = {d[j][0] * nn[j][0], d[j][1] * nn[j][1], d[j][2] * nn[j][2],
+                                         d[j][1] * nn[j][2] + d[j][2] * nn[j][1], d[j][2] * nn[j][0] + d[j][0] * nn[j][2],
+                                         d[j][0] * nn[j][1] + d[j][1] * nn[j][0]};
+                    const double it = 1.0 / tau[j], i1 = 1.0 / s1[j], ghq = gh[j] * qh;
+                    const double ed = eta[j] * dq;
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        x0[k] += b[k] * (k0[j] * it);
+                        x1[k] += b[k] * (iD[j] * ghq * it);
+                        x2[k] += b[k] * (iD[j] * it);
+                        rowC[k] += b[k] * (sg[j] * iD[j] * i1);
+                        rowW[k] += b[k] * (sg[j] * iD[j] * i1 * ed);
+#pragma unroll
+                        for (int m = k; m < 6; ++m) A[6 * k + m] += b[k] * (sg[j] * it * iD[j] * b[m]);
+                    }
+                    cc += iD[j] * ghq * i1;
+                    cw += iD[j] * i1;
+                    c0 += k0[j] * i1;
+                    ww += ed * iD[j] * i1;
+                    wc += ed * iD[j] * ghq * i1;
+                    w0 += ed * (y0[j] + k0[j] * i1);
+                    es += eta[j];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                x0[k] = gsum<L>(x0[k]) - ys[k];
+                x1[k] = gsum<L>(x1[k]);
+                x2[k] = gsum<L>(x2[k]);
+                rowC[k] = gsum<L>(rowC[k]);
+                rowW[k] = gsum<L>(rowW[k]);
+#pragma unroll
+                for (int m = k; m < 6; ++m) {
+                    A[6 * k + m] = gsum<L>(A[6 * k + m]) + S[utri(k, m)];
+                    A[6 * m + k] = A[6 * k + m];
+                }
+            }
+            cc = 1.0 + gsum<L>(cc);
+            cw = gsum<L>(cw);
+            c0 = gsum<L>(c0);
+            ww = 1.0 + gsum<L>(ww);
+            es = gsum<L>(es);
+            wc = gsum<L>(wc) - qh * es;
+            w0 = gsum<L>(w0);
+            int bad = lu6(A);
+            lu6_solve<0>(A, x0);
+            lu6_solve<0>(A, x1);
+            lu6_solve<0>(A, x2);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                cc -= rowC[k] * x1[k];
+                cw -= rowC[k] * x2[k];
+                c0 -= rowC[k] * x0[k];
+                wc -= rowW[k] * x1[k];
+                ww -= rowW[k] * x2[k];
+                w0 -= rowW[k] * x0[k];
+            }
+            const double det = cc * ww - cw * wc;
+            if (det == 0.0) bad = 1;
+            C = (c0 * ww - w0 * cw) / det;
+            Wv = (w0 * cc - c0 * wc) / det;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) ls[k] = x0[k] - C * x1[k] - Wv * x2[k];
+            if (run && bad) {
+                if (lane == 0) atomicMin(errkey, ((unsigned long long)g << 16) | 910ull);
+                run = false;
+            }
+        }
+        // the adjoints of slip resistances and parameters, and abar
+        double abar[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, pb[ADJ_NP] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const int ii = on[j] ? lane + L * j : 0;
+            const double dq = __ldg(sm + ii * ns + ii) - qh;
+            double la = 0.0;
+            if (act[j]) {
+                const double bl = d[j][0] * nn[j][0] * ls[0] + d[j][1] * nn[j][1] * ls[1] + d[j][2] * nn[j][2] * ls[2] +
+                                  (d[j][1] * nn[j][2] + d[j][2] * nn[j][1]) * ls[3] +
+                                  (d[j][2] * nn[j][0] + d[j][0] * nn[j][2]) * ls[4] +
+                                  (d[j][0] * nn[j][1] + d[j][1] * nn[j][0]) * ls[5];
+                la = k0[j] - iD[j] * (sg[j] * bl + gh[j] * qh * C + Wv);
+            }
+            const double c = y0[j] + (act[j] ? la / s1[j] : 0.0), Hj = (qh * C + dq * c) * ag[j];
+            y0[j] = on[j] ? c + dh0[j] * Hj : 0.0;
+            if (act[j]) {
+                pb[0] += la * log(ag[j] / dt);
+                pb[1] += pw[j] * Hj;
+                pb[2] += Hj;
+                pb[3] += dh5[j] * Hj;
+                const double gv = sg[j] * ag[j], lt = la / tau[j];
+                double v[6], vd[3], vn[3];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) v[k] = gv * ls[k] - lt * s[k];
+                const double h = 0.5 * gv;
+                vd[0] = v[0] * nn[j][0] + v[5] * nn[j][1] + v[4] * nn[j][2] + h * (nn[j][1] * rtb[2] - nn[j][2] * rtb[1]);
+                vd[1] = v[5] * nn[j][0] + v[1] * nn[j][1] + v[3] * nn[j][2] + h * (nn[j][2] * rtb[0] - nn[j][0] * rtb[2]);
+                vd[2] = v[4] * nn[j][0] + v[3] * nn[j][1] + v[2] * nn[j][2] + h * (nn[j][0] * rtb[1] - nn[j][1] * rtb[0]);
+                vn[0] = v[0] * d[j][0] + v[5] * d[j][1] + v[4] * d[j][2] + h * (rtb[1] * d[j][2] - rtb[2] * d[j][1]);
+                vn[1] = v[5] * d[j][0] + v[1] * d[j][1] + v[3] * d[j][2] + h * (rtb[2] * d[j][0] - rtb[0] * d[j][2]);
+                vn[2] = v[4] * d[j][0] + v[3] * d[j][1] + v[2] * d[j][2] + h * (rtb[0] * d[j][1] - rtb[1] * d[j][0]);
+                const double *pa = M.ab + ((size_t)mc * M.tld + ii) * 3, *pn = M.an + ((size_t)mc * M.tld + ii) * 3;
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) abar[p][k] += __ldg(pa + p) * vd[k] + __ldg(pn + p) * vn[k];
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                abar[p][k] = gsum<L>(abar[p][k]);
+                if (plastic) abar[p][k] += rxb[p] * rtn[k];
+            }
+        // a sum per increment, so that segments of any length add the same terms
+#pragma unroll
+        for (int k = 0; k < ADJ_NP; ++k) pbar[k] += gsum<L>(pb[k]);
+        if (plastic) abar[2][2] -= dp1 * yph[2];
+        compliance_form<true>(M.e + 9 * mc, a, ls, u, 1.0, abar);
+        if (!plastic) augb[0] = augb[1] = augb[2] = 0.0;
+        angles_bar(ph, a, abar, augb, yph);
+        // the start stress: t = rot^T st rot (TENS_ROT), and -S lambda_s on t
+        {
+            double tb[6], T[3][3], rot[3][3], tmp[3][3], o[3][3];
+            sym6(S, ls, tb);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const int j = (i + 1) % 3, k = (j + 1) % 3;
+                T[i][i] = -tb[i];
+                T[j][k] = -tb[i + 3];
+                T[k][j] = 0.0;
+                rot[j][k] = r[i];
+                rot[k][j] = -r[i];
+                rot[i][i] = sqrt(1.0 - r[j] * r[j] - r[k] * r[k]);
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) tmp[p][k] = rot[p][0] * T[0][k] + rot[p][1] * T[1][k] + rot[p][2] * T[2][k];
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) o[p][k] = tmp[p][0] * rot[k][0] + tmp[p][1] * rot[k][1] + tmp[p][2] * rot[k][2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const int j = (i + 1) % 3, k = (j + 1) % 3;
+                ys[i] = plastic ? o[i][i] : 0.0;
+                ys[i + 3] = plastic ? o[j][k] + o[k][j] : 0.0;
+            }
+        }
+    }
+    if (!run) return;
+#pragma unroll
+    for (int j = 0; j < P; ++j)
+        if (on[j]) g_sv[(size_t)(3 + lane + L * j) * ng + g] = y0[j];
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) g_st[(size_t)k * ng + g] = ys[k];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) g_sv[(size_t)k * ng + g] = yph[k];
+#pragma unroll
+        for (int k = 0; k < ADJ_NP; ++k) g_p[(size_t)k * ng + g] = pbar[k];
+    }
+}
+
+}  // namespace fasdev
