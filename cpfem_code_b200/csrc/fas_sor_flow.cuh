@@ -40,10 +40,10 @@
 // that sweep j + 1 replaced (`old`) are the iterate of sweep j.
 //
 // Measured (first FACSLS, us per sweep, one launch per colour against this
-// kernel): 8-node cubes 8^3 27 / 13.4, 16^3 25 / 13.4, 24^3 31 / 14.6, 32^3
-// 38 / 18.6, 64^3 122 / 83.8 (580 MB of records: 6.9 TB/s of the 7.4 TB/s that
-// a bare ring of copies reaches); FP32 rows 64^3 96.6 / 61.8; 20-node bricks
-// 10^3 60 / 29.7, 21 x 17 x 23 82 / 46.3, 32^3 205 / 144.  A phase of a small mesh
+// kernel): 8-node cubes 8^3 27 / 12.8, 16^3 25 / 12.3, 32^3 38 / 17.0, 64^3 122 /
+// 83.9 (580 MB of records: 6.9 TB/s of the 7.4 TB/s that a bare ring of copies
+// reaches); FP32 rows 64^3 96.6 / 61.8; 20-node bricks 10^3 60 / 28.6, 21 x 17 x
+// 23 82 / 43.1, 32^3 205 / 136.  A phase of a small mesh
 // takes 1.6 us: 0.3 us from the barrier to the published values, 0.9 us until
 // the neighbours hold them, the rest barrier and loop.  Of the 64^3 phase's 10
 // us the copies take 9.4.
@@ -57,9 +57,7 @@
 
 namespace fasdev {
 
-constexpr int FLOW_CW = 12;              // consumer warps
-constexpr int FLOW_HW = 2;               // halo warps
-constexpr int FLOW_SYNC = 32 * (FLOW_CW + FLOW_HW);   // threads of the phase barrier
+constexpr int FLOW_SYNC = 32 * 14;       // threads of the phase barrier: consumer and halo warps (FlowRow)
 constexpr int FLOW_THREADS = FLOW_SYNC + 64;          // + control warp + producer warp: 4 warps and 128
                                                       // registers per thread on each scheduler
 constexpr int FLOW_MAXCOL = 64;
@@ -99,6 +97,14 @@ template <typename T, int S> struct FlowRow {
     static constexpr int MB = LPR * MW * 2;              // bytes of a row's index words
     static constexpr int HQ = S - (SPL - 1) * LPR;       // lane and word of the header: position S
     static constexpr int RPW = 32 / LPR;                 // rows per warp
+    // consumer and halo warps of the fourteen.  A tile polls some tens to hundreds
+    // of pairs a phase, three per FP64 node and one per FP32 node, a pair per thread
+    // and L2 round trip; more halo warps take more of them in one round trip (us per
+    // sweep with 2 / 3 / 4 halo warps: 16^3 13.1 / 12.9 / 12.7, 32^3 18.8 / 17.3 /
+    // 16.8, 64^3 84.3 / 85.1 / 84.1, 20-node 10^3 30.2 / 28.6 / 28.5, 21 x 17 x 23
+    // 46.3 / 43.8 / 42.6, 32^3 144 / 141 / 136; FP32 64^3 61.8 / 61.7 / 62.7).
+    static constexpr int HW = F32 ? 2 : 4;
+    static constexpr int CW = FLOW_SYNC / 32 - HW;
     static constexpr int CH = (S == SLOTS ? 8 : 4) * (F32 ? 2 : 1);   // rows per chunk: about 17 or 25 KB
     static constexpr int EW = F32 ? 10 : 6;              // doubles: rhs 3, 1/diagonal 3 (, base 3, pad)
     static constexpr int EB = EW * 8;
@@ -209,11 +215,11 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
 {
     using L = FlowRow<T, S>;
     constexpr bool F32 = L::F32;
-    constexpr int LPR = L::LPR, SPL = L::SPL;
+    constexpr int LPR = L::LPR, SPL = L::SPL, CW = L::CW, HW = L::HW;
     using XT = std::conditional_t<F32, float, double>;
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ __align__(8) uint64_t s_full[FLOW_MAXSLOT], s_empty[FLOW_MAXSLOT];
-    constexpr int NRED = FLOW_CW * 3;   // shares of a sweep in one CTA
+    constexpr int NRED = CW * 3;   // shares of a sweep in one CTA
     __shared__ double s_red[2][2][NRED];
     __shared__ int s_seg[FLOW_MAXCOL + 1], s_hseg[FLOW_MAXCOL + 1];
     __shared__ volatile int s_cnt, s_verdict, s_conv, s_quit, s_bad, s_go, s_issued;
@@ -266,7 +272,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
     if (s_base < 0) return;      // converged before (a later FP32 cycle), or a wait gave up
     const unsigned long long base = (unsigned)s_base;
 
-    if (warp < FLOW_CW) {
+    if (warp < CW) {
         // ------------------------------------------------------ consumers
         const int row = lane / LPR, q = lane % LPR, lead = lane - q;
         // position / nring by its reciprocal: exact below 2^26 positions
@@ -524,7 +530,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
         int g = s_seg[0] + mine0, c1 = s_seg[1];
         for (int s = 1; s <= A.maxsw; ++s) {
             for (int c = 0; c < ncol; ++c) {
-                for (; g < c1; g += FLOW_CW * L::RPW) {
+                for (; g < c1; g += CW * L::RPW) {
                     if (!taken && !take(g, c1, s, true)) {
                         bad = true;
                         break;
@@ -571,7 +577,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
         if (bad) {
             if (tid == 0) atomicExch(&A.ctl->fault, 1);
         } else {
-            for (int i = tid; i < n; i += 32 * FLOW_CW) {
+            for (int i = tid; i < n; i += 32 * CW) {
                 const int nd = A.node[row0 + i];
 #pragma unroll
                 for (int z = 0; z < 3; ++z)
@@ -579,16 +585,16 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
             }
         }
         if (tid == 0) s_quit = 1;
-    } else if (warp < FLOW_CW + FLOW_HW) {
+    } else if (warp < CW + HW) {
         // ------------------------------------------------------ halo
-        const int hl = tid - 32 * FLOW_CW;
+        const int hl = tid - 32 * CW;
         for (int s = 1; s <= A.maxsw; ++s) {
             const unsigned long long tag = base + (unsigned)s;
             bool bad = false;
             for (int c = 0; c < ncol; ++c) {
                 // one pair per thread: neighbouring pairs share their L2 requests
                 constexpr int W = F32 ? 1 : 3;
-                for (int b = W * s_hseg[c] + hl; b < W * s_hseg[c + 1] && !bad; b += 32 * FLOW_HW) {
+                for (int b = W * s_hseg[c] + hl; b < W * s_hseg[c + 1] && !bad; b += 32 * HW) {
                     const int hb = b / W, z = b - hb * W;
                     XT *y = xs + 3 * (size_t)(n + hb);
                     ulonglong2 v[1];
@@ -606,7 +612,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
             }
             if (bad || s_go) break;
         }
-    } else if (warp == FLOW_CW + FLOW_HW) {
+    } else if (warp == CW + HW) {
         // ------------------------------------------------------ control
         for (int s = 1; s <= A.maxsw; ++s) {
             int it = 0;
