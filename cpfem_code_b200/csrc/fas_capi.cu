@@ -1396,10 +1396,17 @@ template <typename K> unsigned cp_grid(fas_handle *h, K kern, long long n, int *
 }
 
 // Whether the pass runs with a group of lanes per GP (k_cp): the materials
-// allow it and no mode asks for another form.
+// allow it, no mode asks for another form, and the solve takes the assembled
+// rows in FP64.  FP32 rows round them: a difference in the last FP64 bits of a
+// block flips some of these roundings, and the sweeps carry each flip on, so
+// the same update in another order of sums (1e-13 apart) moved the solution of
+// the 64^3 cube by 1.8e-7, as far as the form's own error.  The tuned form's
+// results stay reproducible instead, with one thread per GP: 11 against
+// 2.6 ms a pass at 64^3, of 38 ms an iteration.
 bool group_pass(const fas_handle *h)
 {
-    return h->cp_group && !(h->mode & (FAS_MODE_CP_WARP | FAS_MODE_TANGENT_CONSISTENT));
+    const bool rounded = (h->mode & FAS_MODE_SOR_FP32) && !h->point_mode && !(h->sor_small && !(h->mode & FAS_MODE_SOR_GRID));
+    return h->cp_group && !rounded && !(h->mode & (FAS_MODE_CP_WARP | FAS_MODE_TANGENT_CONSISTENT));
 }
 
 // Scratch and lists of the group pass, allocated with the handle's state.  A
