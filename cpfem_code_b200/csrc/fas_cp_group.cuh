@@ -27,11 +27,12 @@
 // in lockstep, an outer iteration of each at a time.
 //
 // Constitutive pass before and after: 4,096 FCC points 1.75 and 0.20 ms,
-// 100,003 HCP points 5.8 and 2.9 ms, 2^20 FCC points 28.2 and 11.6 ms, a 64^3
-// mesh 11 and 2.6 ms.  The iterations are bound by their dependent chains of
+// 100,003 HCP points 5.8 and 3.1 ms, 2^20 FCC points 28.2 and 12.2 ms, a 64^3
+// mesh 11 and 2.7 ms.  The iterations are bound by their dependent chains of
 // sums, logarithms and divisions (0.3 instructions a cycle and scheduler at 15
 // warps an SM), and by fetching their code.  Against the same update in more
-// digits the error fell from 5e-13 to 4e-14: fewer roundings than elimination.
+// digits the error of the stress and slips fell from 5e-13 to 4e-14: fewer roundings
+// than elimination; that of the hardening increments is PLASTC's (below).
 //
 // The iterations, their stopping tests and error codes are CPSTRS's; sums run
 // in another order and the matrices are solved by the formula, so results equal
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
         // SCALE_IT (amax starts from the first system's am)
         auto scale_it = [&](double top, bool doit) {
             const bool over = doit && top > gamcap;
-            if (!__any_sync(ALL, over)) return;
+            if (!__any_sync(ALL, over)) return false;
             int first = 0x7fffffff, big = 0x7fffffff;
 #pragma unroll
             for (int j = 0; j < P; ++j)
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
                 }
             first = gmin<L>(first);
             big = gmin<L>(big);
-            if (!over) return;
+            if (!over) return false;
             const double3 f = scale_factors(top, gamcap, C.afactor, __ldg(amp + 6 * (big == first || big >= ns ? 0 : big)));
 #pragma unroll
             for (int k = 0; k < 6; ++k) s[k] = f.y * s[k];
@@ -404,6 +405,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
                 lg[j] += f.z;
                 tau[j] = f.y * tau[j];
             }
+            return true;
         };
         scale_it(gammax, run);
         // SLPFTA (crys-cons.f90:24-128): Newton on the logarithms of the active
@@ -496,7 +498,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
         }
         w = gsum<L>(w);
         if (gisum<L>(zero ? 1 : 0) != 0 && run && !rc) rc = 910;
-        scale_it(gmax<L>(top), run && !rc);
+        const bool scaled = scale_it(gmax<L>(top), run && !rc);
         // plastic strain, djac = b X^-1 b^T + S and the strain error
         double deff, em, A[36];
         bool fin;
@@ -568,6 +570,33 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_cp(DevMat M, DevCtrl C, DevGp
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) rtn[k] = gsum<L>(rtn[k]);
+        // The hardening increments s1 - s0 that are kept: where the slips are small
+        // they are a few thousand roundings of s0, and the order of the sum shows in
+        // their seventh to ninth digit.  So s1 is added up once more in PLASTC's order
+        // (ela-plas.f90:110-201), system by system onto s0.  SCALE_IT in a point's
+        // last iteration, which changes the slips after PLASTC, leaves it as it is.
+        {
+            double sq[P], hd[P];
+#pragma unroll
+            for (int k = 0; k < P; ++k) {
+                sq[k] = s0[k];
+                const int ii = on[k] ? lane + L * k : 0;
+                hd[k] = __ldg(sm + ii * ns + ii) * gh[k];
+            }
+#pragma unroll
+            for (int k = 0; k < P; ++k) {
+                const double hq = on[k] ? q * gh[k] : 0.0, ag = fabs(gam[k]);
+#pragma unroll
+                for (int l = 0; l < L; ++l) {
+                    const double h = __shfl_sync(ALL, hq, l, L), a = __shfl_sync(ALL, ag, l, L);
+#pragma unroll
+                    for (int m = 0; m < P; ++m) sq[m] = fma(m == k && l == lane ? hd[m] : h, a, sq[m]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < P; ++k)
+                if (!scaled) s1[k] = sq[k];
+        }
         if (fin) {
             if (lane == 0) {
                 G.cp_iters[g] = rc && W.stress ? -1 : iter;
