@@ -175,6 +175,10 @@ struct fas_handle {
     DVec<unsigned char> fl_rec64, fl_rec32;   // the chunks' records
     DVec<double> fl_old;
     DVec<ulonglong2> fl_sync;    // published values, then the tiles' shares
+    bool fl_cluster = false;     // the tiles are one thread-block cluster
+    DVec<uint16_t> fl_pptr;      // ... where each row's destinations begin
+    DVec<unsigned> fl_pdst;
+    DVec<int> fl_pfirst;
     // NRITER of an increment as one CUDA graph (FAS_MODE_GRAPH): loop state,
     // report lines, the instantiated graph of each increment, and the two
     // side streams its nested loop bodies are captured on
@@ -595,16 +599,17 @@ void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::v
 }
 
 // Tile layout of the persistent SOR solve (k_sor_flow): one spatial tile of
-// nodes per CTA, its rows by colour (rows that other tiles read first), the
+// nodes per CTA (one tile, a cluster of 16 or one per SM, by the rows' bytes), its rows by colour (rows that other tiles read first), the
 // tile-local index of every column, and the halo: the nodes of other tiles
 // that the tile's rows read, by colour.  A mesh with more colours than the
 // kernel's tables, or tiles whose solution values leave no room for a copy
 // ring (about 90^3 8-node bricks per GPU in FP64), keeps the colour kernels.
-template <typename T, int S> bool flow_fits(int n, int nh)
+template <typename T, int S> bool flow_fits(int n, int nh, int ndst)
 {
     using L = FlowRow<T, S>;
     size_t o = L::F32 ? (size_t)n * 24 + (size_t)(n + nh) * 12 : (size_t)(n + nh) * 24;
-    o += (size_t)nh * 4 + (S == SLOTS ? 0 : (size_t)((n + L::CH - 1) / L::CH + 1) * 4);
+    o += ndst >= 0 ? FLOW_CL_BYTES + (size_t)ndst * 4 + (size_t)(n + 1) * 2 : (size_t)nh * 4;
+    o += (S == SLOTS ? 0 : (size_t)((n + L::CH - 1) / L::CH + 1) * 4);
     o = (o + 127) & ~(size_t)127;
     return n + nh < 65536 && o + 3 * (size_t)L::SLOT <= (size_t)FLOW_SMEM;
 }
@@ -615,10 +620,20 @@ template <typename F> auto flow_shape(int slots, F &&f)
     return slots == SLOTS ? f(std::integral_constant<int, SLOTS>{}) : f(std::integral_constant<int, SLOTS20>{});
 }
 
-// Bytes of FP64 rows up to which the solve runs as one tile: one SM then
-// needs no exchange with others, and its phases (a CTA barrier each) stay
-// shorter than the 0.5 us an exchange takes.
-constexpr long long FLOW_ONE_TILE_BYTES = 700 * 1024;
+// Bytes of packed FP64 rows up to which the solve runs as one tile: the rows of
+// more lie partly outside one SM's shared memory, and its ten consumer warps
+// need several rounds a phase.  us per sweep as one tile, as a cluster of 16 and
+// as one tile per SM: 3^3 8-node bricks (127 KB) 6.3 / 7.2 / 9.0, 4^3 (248 KB) 8.0 /
+// 8.0 / 10.7, 5^3 (428 KB) 10.9 / 8.5 / 10.8; 20-node bricks 2^3 (340 KB) 16.5 / 18.8 /
+// 22.3, 3^3 (0.9 MB) - / 19.3 / 27.5.
+constexpr long long FLOW_ONE_TILE_BYTES = 350 * 1024;
+// Bytes of packed FP64 rows up to which the tiles are one cluster of 16 CTAs,
+// whose exchange is shorter but whose 16 SMs stream what 3.3 MB of shared memory
+// do not hold.  us per sweep as a cluster and as one tile per SM: 8-node bricks
+// 8^3 9.1 / 11.3, 12^3 (4.4 MB) 11.2 / 11.8, 14^3 (6.7 MB) 13.6 / 11.6; 20-node bricks
+// 5^3 23.7 / 27.4, 6^3 (5.2 MB) 24.6 / 28.5, 8^3 (11 MB) 29.9 / 28.2; FP32 rows 12^3
+// 12.7 / 15.3, 20-node 6^3 33.5 / 36.5.
+constexpr long long FLOW_CLUSTER_BYTES = 5632 * 1024;
 // Rows per tile up to which every colour is cut evenly by itself: phases of a
 // few rows are as long as their largest share (us per sweep evenly against
 // by position: 32^3 18.4 against 19.7, 21 x 17 x 23 20-node bricks 46.9
@@ -628,14 +643,55 @@ constexpr long long FLOW_EVEN_ROWS = 512;
 // Rows per tile below which a mesh gets fewer tiles than SMs.
 constexpr int FLOW_MIN_ROWS = 16;
 
+// The launch of k_sor_flow: a cooperative grid of one CTA per tile, or one cluster.
+struct FlowLaunch {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = {};
+    FlowLaunch(int ntiles, bool cluster, cudaStream_t s)
+    {
+        if (cluster) {
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = ntiles;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        } else {
+            at[0].id = cudaLaunchAttributeCooperative;
+            at[0].val.cooperative = 1;
+        }
+        cfg.gridDim = dim3(ntiles);
+        cfg.blockDim = dim3(FLOW_THREADS);
+        cfg.dynamicSmemBytes = FLOW_SMEM;
+        cfg.stream = s;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    FlowLaunch(const FlowLaunch &) = delete;
+};
+
+// Whether the device holds a cluster of FLOW_CLUSTER CTAs of every form.
+bool flow_cluster_fits(fas_handle *h)
+{
+    return flow_shape(h->slots, [&](auto sl) {
+        auto fits = [&](auto kern) {
+            FlowLaunch l(FLOW_CLUSTER, true, h->stream);
+            int n = 0;
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kern, &l.cfg);
+            if (e != cudaSuccess) cudaGetLastError();
+            return e == cudaSuccess && n >= 1;
+        };
+        return fits(&k_sor_flow<double, sl(), true>) && fits(&k_sor_flow<float, sl(), true>);
+    });
+}
+
 int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<int> &bcol_host,
                const std::vector<int> &nslot_host, const std::vector<int> &rowof_host)
 {
     if (h->ncol > FLOW_MAXCOL) return 0;
     const int nn = h->nnod, ncol = h->ncol, S = h->slots, crow = crow_of(S);
-    const int nt = (long long)nn * brow_of(S) * 8 <= FLOW_ONE_TILE_BYTES
-                       ? 1
-                       : std::min(h->nsm, std::max(1, nn / FLOW_MIN_ROWS));
+    long long bytes = 0;         // of the rows as FlowRow packs them
+    for (int p = 0; p < nn; ++p) bytes += S == SLOTS ? FlowRow<double, SLOTS>::VB : 72LL * nslot_host[p];
+    const bool one = bytes <= FLOW_ONE_TILE_BYTES;
+    const bool cluster = !one && bytes <= FLOW_CLUSTER_BYTES && nn >= FLOW_CLUSTER && flow_cluster_fits(h);
+    const int nt = one ? 1 : cluster ? FLOW_CLUSTER : std::min(h->nsm, std::max(1, nn / FLOW_MIN_ROWS));
     std::vector<int> nodes(nn), tile_of(nn, 0), clo(h->col_start.begin(), h->col_start.end() - 1),
         chi(h->col_start.begin() + 1, h->col_start.end());
     for (int m = 0; m < nn; ++m) nodes[rowof_host[m]] = m;   // by colour
@@ -679,6 +735,7 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
         early = nl <= most;
     }
     bool ok64 = true, ok32 = true;
+    std::vector<std::vector<unsigned>> dests(cluster ? nn : 0);   // of every row: the halo entries that hold its node
     for (int t = 0; t < nt; ++t) {
         const int n = trow[t + 1] - trow[t];
         halo.clear();
@@ -706,9 +763,13 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
             hidx[halo[k]] = n + k;
             hrow.push_back(rowt[halo[k]]);
         }
-        ok64 = ok64 && flow_shape(S, [&](auto s) { return flow_fits<double, s()>(n, nh); });
-        ok32 = ok32 && flow_shape(S, [&](auto s) { return flow_fits<float, s()>(n, nh); });
-        if (!ok64 && !ok32) return 0;
+        if (cluster) {
+            for (int k = 0; k < nh; ++k) dests[hrow[hptr[t] + k]].push_back((unsigned)t << 16 | (unsigned)(n + k));
+        } else {
+            ok64 = ok64 && flow_shape(S, [&](auto s) { return flow_fits<double, s()>(n, nh, -1); });
+            ok32 = ok32 && flow_shape(S, [&](auto s) { return flow_fits<float, s()>(n, nh, -1); });
+            if (!ok64 && !ok32) return 0;
+        }
         for (int r = trow[t]; r < trow[t + 1]; ++r) {
             const int p = src[r], ns = nslot_host[p];
             const int *c = &bcol_host[(size_t)p * crow];
@@ -725,6 +786,23 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
                 lcol[(size_t)r * S + at] = (uint16_t)(tile_of[c[sl]] == t ? rowt[c[sl]] - trow[t] : hidx[c[sl]]);
             }
         }
+    }
+    // the cluster's destinations: [tile] its rows' first ones and its end, tile-local
+    std::vector<uint16_t> pptr;
+    std::vector<unsigned> pdst;
+    std::vector<int> pfirst(1, 0);
+    for (int t = 0; t < nt && cluster; ++t) {
+        for (int r = trow[t]; r < trow[t + 1]; ++r) {
+            pptr.push_back((uint16_t)(pdst.size() - pfirst[t]));
+            pdst.insert(pdst.end(), dests[r].begin(), dests[r].end());
+        }
+        const int n = trow[t + 1] - trow[t], nh = hptr[t + 1] - hptr[t], ndst = (int)pdst.size() - pfirst[t];
+        pptr.push_back((uint16_t)ndst);
+        pfirst.push_back((int)pdst.size());
+        if (ndst >= 65536) return 0;
+        ok64 = ok64 && flow_shape(S, [&](auto s) { return flow_fits<double, s()>(n, nh, ndst); });
+        ok32 = ok32 && flow_shape(S, [&](auto s) { return flow_fits<float, s()>(n, nh, ndst); });
+        if (!ok64 && !ok32) return 0;
     }
     // value offsets of 81-slot rows, packed to their own slot counts
     std::vector<unsigned> vo64(nn + 1, 0), vo32(nn + 1, 0);
@@ -766,9 +844,13 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
     if (!rc) rc = up(h->fl_from, from);
     if (!rc && S != SLOTS) rc = up(h->fl_voff64, vo64);
     if (!rc && S != SLOTS) rc = up(h->fl_voff32, vo32);
+    if (!rc && cluster) rc = up(h->fl_pptr, pptr);
+    if (!rc && cluster) rc = up(h->fl_pdst, pdst);
+    if (!rc && cluster) rc = up(h->fl_pfirst, pfirst);
     if (rc) return rc;
     CK(cudaStreamSynchronize(s));
     h->fl_nt = nt;
+    h->fl_cluster = cluster;
     h->fl_early = early;
     h->fl_ok64 = ok64;
     h->fl_ok32 = ok32;
@@ -911,11 +993,17 @@ int create_impl(fas_handle *h, const fas_mesh_desc *Md, const fas_matl_desc *T, 
                             cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem_bytes<float, SLOTS_SYM>()));
     for (int slots : {SLOTS, SLOTS20})
         CK(flow_shape(slots, [](auto sl) {
-            const cudaError_t e =
-                cudaFuncSetAttribute(k_sor_flow<double, sl()>, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
-            return e != cudaSuccess
-                       ? e
-                       : cudaFuncSetAttribute(k_sor_flow<float, sl()>, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
+            cudaError_t e = cudaSuccess;
+            auto set = [&](auto kern, bool cluster) {
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM);
+                if (e == cudaSuccess && cluster)
+                    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            };
+            set(&k_sor_flow<double, sl()>, false);
+            set(&k_sor_flow<float, sl()>, false);
+            set(&k_sor_flow<double, sl(), true>, true);
+            set(&k_sor_flow<float, sl(), true>, true);
+            return e;
         }));
     CK(cudaMallocHost((void **)&h->hc, sizeof(HostCtl)));
     CK(cudaEventCreate(&h->ev_t0));
@@ -1897,11 +1985,11 @@ template <typename T> int flow_begin(fas_handle *h, const BlockDev &B)
     kern<<<blk, 256, 0, h->stream>>>(B, h->fl_src.p, FlowBufs<T>::voff(h), h->fl_tile.p, h->fl_trow.p,
                                      FlowBufs<T>::cptr(h), h->fl_from.p, h->rhs.p, FlowBufs<T>::rec(h).p);
     LAUNCHED(h);
-    CK(h->fl_sync.zero(h->stream));
+    if (!h->fl_cluster) CK(h->fl_sync.zero(h->stream));
     return 0;
 }
 
-// One cooperative launch: at most maxsw sweeps from zero, the result in
+// One launch: at most maxsw sweeps from zero, the result in
 // `sol`, sweeps counted on from ctl->sweeps.
 template <typename T> int launch_flow(fas_handle *h, double *sol, int maxsw, double tolerl)
 {
@@ -1925,17 +2013,15 @@ template <typename T> int launch_flow(fas_handle *h, double *sol, int maxsw, dou
     a.maxsw = maxsw;
     a.early = h->fl_early ? 1 : 0;
     a.tolerl = tolerl;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(h->fl_nt);
-    cfg.blockDim = dim3(FLOW_THREADS);
-    cfg.dynamicSmemBytes = FLOW_SMEM;
-    cfg.stream = h->stream;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, flow_shape(h->slots, [](auto sl) { return &k_sor_flow<T, sl()>; }), a));
+    a.pptr = h->fl_pptr.p;
+    a.pdst = h->fl_pdst.p;
+    a.pfirst = h->fl_pfirst.p;
+    FlowLaunch l(h->fl_nt, h->fl_cluster, h->stream);
+    CK(cudaLaunchKernelEx(&l.cfg,
+                          flow_shape(h->slots, [&](auto sl) {
+                              return h->fl_cluster ? &k_sor_flow<T, sl(), true> : &k_sor_flow<T, sl(), false>;
+                          }),
+                          a));
     LAUNCHED(h);
     return 0;
 }

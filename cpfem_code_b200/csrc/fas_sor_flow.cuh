@@ -21,6 +21,11 @@
 //     cycles from one SM's store to another SM's register, about a third of
 //     a kernel boundary).
 //
+// Meshes of a few MB run as one thread-block cluster of 16 tiles (CL): a value
+// goes from the registers of the row's lanes into the shared memory of each tile
+// that reads it (st.async), and the barrier of its colour there counts the
+// bytes, so nothing is polled.  The smallest run as one tile.
+//
 // Order.  Rows of a tile are ordered by colour, those that other tiles need
 // first.  In phase c the consumer warps update the tile's rows of colour c
 // while the halo warps fetch the neighbours' nodes of colour c; one CTA
@@ -30,7 +35,10 @@
 // one-launch-per-colour SOR.  A published value is overwritten in place:
 // the owner updates node n in sweep s + 1 only after it has fetched the
 // values of all of n's neighbours that were computed from n's value of
-// sweep s, so every reader has taken it (the pattern is symmetric).
+// sweep s, so every reader has taken it (the pattern is symmetric).  The same
+// holds for a value stored into another tile's shared memory, and for its
+// colour's barrier: the bytes of sweep s + 1 start to come only after every
+// warp of that tile has passed the phase of sweep s.
 //
 // Stopping test.  Each tile publishes its share of |x_s - x_(s-1)|^2 and
 // |x_s|^2 the same way; the control warp of every tile sums all shares in
@@ -40,13 +48,15 @@
 // that sweep j + 1 replaced (`old`) are the iterate of sweep j.
 //
 // Measured (first FACSLS, us per sweep, one launch per colour against this
-// kernel): 8-node cubes 8^3 27 / 12.8, 16^3 25 / 12.3, 32^3 38 / 17.0, 64^3 122 /
-// 83.9 (580 MB of records: 6.9 TB/s of the 7.4 TB/s that a bare ring of copies
-// reaches); FP32 rows 64^3 96.6 / 61.8; 20-node bricks 10^3 60 / 28.6, 21 x 17 x
-// 23 82 / 43.1, 32^3 205 / 136.  A phase of a small mesh
-// takes 1.6 us: 0.3 us from the barrier to the published values, 0.9 us until
-// the neighbours hold them, the rest barrier and loop.  Of the 64^3 phase's 10
-// us the copies take 9.4.
+// kernel): 8-node cubes 3^3 - / 6.3 (one tile), 8^3 27 / 9.0 (cluster; 11.3 as one
+// tile per SM), 12^3 - / 11.2 (11.8), 16^3 25 / 11.8, 32^3 38 / 16.5, 64^3 122 / 83.9 (580
+// MB of records: 6.9 TB/s of the 7.4 TB/s that a bare ring of copies reaches);
+// FP32 rows 64^3 96.6 / 61.8; 20-node bricks 4^3 - / 21.5 (27.9), 10^3 60 / 28.5, 21 x
+// 17 x 23 82 / 45.7, 32^3 205 / 136.  A phase of one tile per SM takes 1.4 us on a
+// small mesh: 0.3 us from the barrier to the published values, 0.9 us until the
+// neighbours hold them; of a cluster 1.1 us, of one tile 0.8 us, most of it the
+// dependent FP64 chain from the late columns to the point update.  Of the 64^3
+// phase's 10 us the copies take 9.4.
 //
 // Every wait is bounded.  A wait that gives up raises ctl->fault; a CTA
 // leaves only at a barrier where all its warps agree, after its own copies
@@ -64,6 +74,13 @@ constexpr int FLOW_MAXCOL = 64;
 constexpr int FLOW_MAXSLOT = 64;         // chunk slots in shared memory
 constexpr int FLOW_SMEM = 223 * 1024;    // dynamic part (about 3 KB is static, of 227 KB)
 constexpr int FLOW_RING_BYTES = 112 * 1024;   // copies in flight that cover HBM's latency at full rate
+// The cluster form: at most 16 tiles, one cluster.  Its control block lies at
+// the start of every CTA's dynamic shared memory, at the same offsets: one
+// barrier per colour for the halo's bytes, one per slot of the shares, and the
+// shares of four sweeps.
+constexpr int FLOW_CLUSTER = 16;
+constexpr int FLOW_CL_PBAR = FLOW_MAXCOL * 8, FLOW_CL_PART = FLOW_CL_PBAR + 32,
+              FLOW_CL_BYTES = (FLOW_CL_PART + 4 * FLOW_CLUSTER * 16 + 127) & ~127;
 
 // Row format of S slots in value type T.  LPR lanes serve a row, lane q the
 // positions q, q + LPR, ...
@@ -133,6 +150,9 @@ template <typename T> struct FlowArgs {
     const int *node;             // [R]
     ulonglong2 *gx;              // published values: FP64 [R][3] {value, sweep}, FP32 [R] {x, y, z, sweep}
     ulonglong2 *part;            // [4][ntiles][2] {share, sweep}
+    const uint16_t *pptr;        // cluster form: [R + ntiles] a row's first destination, tile-local, and each tile's end
+    const unsigned *pdst;        // tile << 16 | index of the node's values there
+    const int *pfirst;           // [ntiles + 1] first destination of a tile
     double *old;                 // [R][3] the value that the last update replaced
     double *sol;                 // result, node order
     SorCtl *ctl;
@@ -210,7 +230,54 @@ template <int N> __device__ __forceinline__ bool flow_poll(const ulonglong2 *p, 
     return false;
 }
 
-template <typename T, int S>
+// Cluster form: a value into another CTA's shared memory, counted in bytes by a
+// barrier there.
+__device__ __forceinline__ unsigned cl_addr(unsigned addr, unsigned rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cl_push(unsigned addr, double v, unsigned bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cl_push(unsigned addr, float v, unsigned bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+                 "r"(__float_as_uint(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cl_push2(unsigned addr, double a, double b, unsigned bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(bar)
+                 : "memory");
+}
+// every thread of every CTA of the cluster
+__device__ __forceinline__ void cl_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// Waits for a phase of a barrier that other CTAs complete: at most two seconds,
+// and not once another CTA has raised the fault.
+__device__ __forceinline__ bool cl_wait(uint64_t *bar, unsigned parity, const SorCtl *ctl)
+{
+    unsigned long long t0 = 0;
+    for (int it = 0;; ++it) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((it & 63) == 63) {
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+            if (t0 == 0) t0 = now;
+            if (now - t0 > 2000000000ull || ((volatile const SorCtl *)ctl)->fault) return false;
+        }
+    }
+}
+
+template <typename T, int S, bool CL = false>
 __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> A)
 {
     using L = FlowRow<T, S>;
@@ -228,16 +295,24 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
     const int ncol = A.ncol, row0 = A.trow[t], n = A.trow[t + 1] - row0;
     const int h0 = A.hptr[t], nh = A.hptr[t + 1] - h0;
     const int nch = (n + L::CH - 1) / L::CH;
-    // shared memory: own values, halo values, halo rows, chunk offsets, slots
-    size_t o = 0;
-    double *xd = reinterpret_cast<double *>(dyn);            // FP64: own + halo; FP32: own only
+    // shared memory: (control block,) own values, halo values, halo rows or
+    // destinations, chunk offsets, slots
+    size_t o = CL ? FLOW_CL_BYTES : 0;
+    uint64_t *s_hal = reinterpret_cast<uint64_t *>(dyn), *s_pbar = reinterpret_cast<uint64_t *>(dyn + FLOW_CL_PBAR);
+    double2 *s_part = reinterpret_cast<double2 *>(dyn + FLOW_CL_PART);
+    double *xd = reinterpret_cast<double *>(dyn + o);        // FP64: own + halo; FP32: own only
     o += (size_t)(F32 ? n : n + nh) * 24;
-    XT *xs = F32 ? reinterpret_cast<XT *>(dyn + o) : reinterpret_cast<XT *>(dyn);
+    XT *xs = F32 ? reinterpret_cast<XT *>(dyn + o) : reinterpret_cast<XT *>(xd);
     if (F32) o += (size_t)(n + nh) * 12;
     int *s_hrow = reinterpret_cast<int *>(dyn + o);
-    o += (size_t)nh * 4;
+    const int d0 = CL ? A.pfirst[t] : 0, nd = CL ? A.pfirst[t + 1] - d0 : 0;
+    unsigned *s_pdst = reinterpret_cast<unsigned *>(dyn + o);
+    if (CL) o += (size_t)nd * 4;
+    else o += (size_t)nh * 4;
     unsigned *s_coff = reinterpret_cast<unsigned *>(dyn + o);
     if (S != SLOTS) o += (size_t)(nch + 1) * 4;
+    uint16_t *s_pptr = reinterpret_cast<uint16_t *>(dyn + o);
+    if (CL) o += (size_t)(n + 1) * 2;
     o = (o + 127) & ~(size_t)127;
     unsigned char *slots = dyn + o;
     const int nslots = min(FLOW_MAXSLOT, (int)((FLOW_SMEM - o) / L::SLOT));
@@ -261,7 +336,17 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
     for (int i = tid; i < (F32 ? n : n + nh) * 3; i += FLOW_THREADS) xd[i] = 0.0;
     if (F32)
         for (int i = tid; i < (n + nh) * 3; i += FLOW_THREADS) xs[i] = (XT)0;
-    for (int i = tid; i < nh; i += FLOW_THREADS) s_hrow[i] = A.hrow[h0 + i];
+    if constexpr (CL) {
+        // where the destinations lie in their CTA's shared memory, above its number
+        for (int i = tid; i < nd; i += FLOW_THREADS) {
+            const unsigned w = A.pdst[d0 + i], rk = w >> 16;
+            const unsigned own = F32 ? 24u * (unsigned)(A.trow[rk + 1] - A.trow[rk]) : 0u;
+            s_pdst[i] = rk << 20 | (FLOW_CL_BYTES + own + 3u * sizeof(XT) * (w & 0xffffu));
+        }
+        for (int i = tid; i <= n; i += FLOW_THREADS) s_pptr[i] = A.pptr[row0 + t + i];
+    } else {
+        for (int i = tid; i < nh; i += FLOW_THREADS) s_hrow[i] = A.hrow[h0 + i];
+    }
     for (int i = tid; i <= ncol; i += FLOW_THREADS) {
         s_seg[i] = A.seg[t * (ncol + 1) + i];
         s_hseg[i] = A.hseg[t * (ncol + 1) + i];
@@ -270,6 +355,21 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
         for (int i = tid; i <= nch; i += FLOW_THREADS) s_coff[i] = A.voff[row0 + min(n, i * L::CH)];
     __syncthreads();
     if (s_base < 0) return;      // converged before (a later FP32 cycle), or a wait gave up
+    if constexpr (CL) {
+        if (tid < ncol) {
+            mbar_init(&s_hal[tid], 1);
+            mbar_fence_init();
+            if (s_hseg[tid + 1] > s_hseg[tid])
+                mbar_expect_tx(&s_hal[tid], (unsigned)(s_hseg[tid + 1] - s_hseg[tid]) * 3u * sizeof(XT));
+        } else if (tid >= FLOW_MAXCOL && tid < FLOW_MAXCOL + 4) {
+            mbar_init(&s_pbar[tid - FLOW_MAXCOL], 1);
+            mbar_fence_init();
+            mbar_expect_tx(&s_pbar[tid - FLOW_MAXCOL], 16u * A.ntiles);
+        }
+        __syncthreads();
+        cl_sync();               // every CTA's barriers and zeros stand
+    }
+    const unsigned dyn0 = smem_u32(dyn);
     const unsigned long long base = (unsigned)s_base;
 
     if (warp < CW) {
@@ -420,7 +520,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
             }
             return true;
         };
-        auto finish = [&](int sw) {
+        auto finish = [&](int sw, int c) {
             double a0, a1, a2, x0, x1, x2;
             if constexpr (F32) {
                 // FP32 products and lane sums in slot order, joined in FP64, and the
@@ -509,7 +609,15 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
             const double xq = F32 ? tq : oq + tq, dq = F32 ? tq - oq : tq;
             const bool mine = live && q < 3;
             const size_t r = (size_t)row0 + i;
-            if constexpr (F32)
+            if constexpr (CL) {
+                if (pub && mine) {
+                    const int k1 = s_pptr[i + 1];
+                    for (int k = s_pptr[i]; k < k1; ++k) {
+                        const unsigned w = s_pdst[k], rk = w >> 20;
+                        cl_push(cl_addr(dyn0 + (w & 0xfffffu) + (unsigned)sizeof(XT) * q, rk), (XT)xq, cl_addr(dyn0 + 8u * c, rk));
+                    }
+                }
+            } else if constexpr (F32)
                 st_pair_if(pub && mine && q == 0, A.gx + r,
                            (unsigned long long)__float_as_uint((float)x0) |
                                ((unsigned long long)__float_as_uint((float)x1) << 32),
@@ -526,8 +634,11 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
             }
         };
         bool taken = false;
-        const int mine0 = warp * L::RPW;
-        int g = s_seg[0] + mine0, c1 = s_seg[1];
+        // A phase's groups begin at the warp after the last one of the phase
+        // before, so that the warps of a phase of few rows have taken their rows
+        // while others finished the phase before (us per sweep with every phase
+        // beginning at warp 0: clusters 8^3 11.0, 20-node 4^3 27.9 against 9.0, 21.5).
+        int w0 = 0, g = s_seg[0] + warp * L::RPW, c1 = s_seg[1];
         for (int s = 1; s <= A.maxsw; ++s) {
             for (int c = 0; c < ncol; ++c) {
                 for (; g < c1; g += CW * L::RPW) {
@@ -536,7 +647,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
                         break;
                     }
                     taken = false;
-                    finish(s);
+                    finish(s, c);
                 }
                 const bool last = c + 1 == ncol;
                 if (last) {
@@ -558,7 +669,8 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
                     }
                 }
                 const int cn = last ? 0 : c + 1, sn = last ? s + 1 : s;
-                g = s_seg[cn] + mine0;
+                w0 = (w0 + (c1 - s_seg[c] + L::RPW - 1) / L::RPW) % CW;
+                g = s_seg[cn] + (warp - w0 + (warp < w0 ? CW : 0)) * L::RPW;
                 c1 = s_seg[cn + 1];
                 if (L::AHEAD && A.early && !bad && g < c1 && sn <= A.maxsw) {
                     __syncwarp();
@@ -592,6 +704,18 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
             const unsigned long long tag = base + (unsigned)s;
             bool bad = false;
             for (int c = 0; c < ncol; ++c) {
+                if constexpr (CL) {
+                    const int nc = s_hseg[c + 1] - s_hseg[c];
+                    if (nc > 0) {
+                        bad = !cl_wait(&s_hal[c], (unsigned)(s - 1) & 1u, A.ctl);
+                        // no value of the next sweep's colour c completes its phase before
+                        // this: the barrier's one arrival is still to come
+                        if (hl == 0 && !bad) mbar_expect_tx(&s_hal[c], (unsigned)nc * 3u * sizeof(XT));
+                    }
+                    bad = flow_bar_or(bad);
+                    if (bad) break;
+                    continue;
+                }
                 // one pair per thread: neighbouring pairs share their L2 requests
                 constexpr int W = F32 ? 1 : 3;
                 for (int b = W * s_hseg[c] + hl; b < W * s_hseg[c + 1] && !bad; b += 32 * HW) {
@@ -632,19 +756,32 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
                 a += __shfl_xor_sync(0xffffffffu, a, u);
                 b += __shfl_xor_sync(0xffffffffu, b, u);
             }
-            ulonglong2 *ps = A.part + (size_t)(s & 3) * A.ntiles * 2;
-            const unsigned long long tag = base + (unsigned)s;
-            if (lane == 0) {
-                st_pair(ps + 2 * t, __double_as_longlong(a), tag);
-                st_pair(ps + 2 * t + 1, __double_as_longlong(b), tag);
-            }
             bool ok = true;
-            a = b = 0.0;
-            for (int j = lane; j < A.ntiles && ok; j += 32) {
-                ulonglong2 v[2];
-                ok = flow_poll<2>(ps + 2 * j, tag, 0, A.ctl, v);
-                a += __longlong_as_double(v[0].x);
-                b += __longlong_as_double(v[1].x);
+            if constexpr (CL) {
+                const int sl = s & 3;
+                if (lane < A.ntiles)
+                    cl_push2(cl_addr(dyn0 + FLOW_CL_PART + 16u * (unsigned)(sl * FLOW_CLUSTER + t), lane), a, b,
+                             cl_addr(dyn0 + FLOW_CL_PBAR + 8u * sl, lane));
+                // the k-th use of slot sl, k = (s - 1) / 4 from sweep 1 on
+                ok = cl_wait(&s_pbar[sl], (unsigned)((s - 1) >> 2) & 1u, A.ctl);
+                const double2 v = lane < A.ntiles ? s_part[sl * FLOW_CLUSTER + lane] : make_double2(0.0, 0.0);
+                a = v.x, b = v.y;
+                __syncwarp();
+                if (lane == 0 && ok) mbar_expect_tx(&s_pbar[sl], 16u * A.ntiles);
+            } else {
+                ulonglong2 *ps = A.part + (size_t)(s & 3) * A.ntiles * 2;
+                const unsigned long long tag = base + (unsigned)s;
+                if (lane == 0) {
+                    st_pair(ps + 2 * t, __double_as_longlong(a), tag);
+                    st_pair(ps + 2 * t + 1, __double_as_longlong(b), tag);
+                }
+                a = b = 0.0;
+                for (int j = lane; j < A.ntiles && ok; j += 32) {
+                    ulonglong2 v[2];
+                    ok = flow_poll<2>(ps + 2 * j, tag, 0, A.ctl, v);
+                    a += __longlong_as_double(v[0].x);
+                    b += __longlong_as_double(v[1].x);
+                }
             }
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) s_bad = 1;
@@ -705,6 +842,15 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
         for (int k = 0; k < nres; ++k) mbar_wait_bounded(&s_full[k], 0u);
         for (int j = max(0, issued - nring); j < issued; ++j)
             mbar_wait_bounded(&s_full[nres + j % nring], (unsigned)((j / nring) & 1));
+    }
+    if constexpr (CL) {
+        // No CTA leaves while another may still write to it.  A solve that ends
+        // has waited for every value sent to it; one that gave up leaves some in
+        // flight, so its CTAs wait a millisecond, where a value takes less than
+        // a microsecond.
+        cl_sync();
+        if (((volatile const SorCtl *)A.ctl)->fault)
+            for (int k = 0; k < 1000; ++k) __nanosleep(1000);
     }
 }
 

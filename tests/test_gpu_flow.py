@@ -71,3 +71,29 @@ def test_flow_equals_colour_launches(n, nodes, extra, fp32):
         np.testing.assert_array_equal(got[0], got[1])
     finally:
         g.close()
+
+
+# both sides of the limits between one tile, a cluster of 16 tiles and a tile
+# per SM (180 and 2,906 rows of 27 slots; 350 KB and 5.5 MB of 81-slot rows), and
+# far ties inside a cluster; each size also as a whole increment in one graph
+CLUSTER = [((4, 4, 5), 8, {}), ((5, 5, 5), 8, {}), ((13, 13, 13), 8, {}), ((13, 13, 14), 8, {}), ((3, 2, 2), 20, {}),
+           ((6, 6, 6), 20, {}), ((7, 7, 6), 20, {}), ((5, 4, 4), 8, dict(ties=(True, True, True)))]
+
+
+@pytest.mark.parametrize("n,nodes,extra", CLUSTER)
+@pytest.mark.parametrize("fp32", [False, True])
+def test_flow_at_the_limits_of_its_forms(n, nodes, extra, fp32):
+    test_flow_equals_colour_launches(n, nodes, extra, fp32)
+
+
+@pytest.mark.parametrize("n", [(2, 3, 2), (6, 5, 6)])
+def test_flow_forms_in_graphs(n):
+    p = generator.structured_cube(n=n, ninc=1, seed=5, xfree=1)
+    out = []
+    for mode in (abi.FAS_MODE_PLAIN, abi.FAS_MODE_GRAPH):
+        g = GpuSolver(p.copy(), mode=mode)
+        g.increment(1)
+        out.append(g.download(p.copy()))
+        g.close()
+    np.testing.assert_array_equal(out[0].x, out[1].x)
+    np.testing.assert_array_equal(out[0].st, out[1].st)
