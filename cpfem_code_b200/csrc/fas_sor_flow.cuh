@@ -52,7 +52,7 @@
 // tile per SM), 12^3 - / 11.2 (11.8), 16^3 25 / 11.8, 32^3 38 / 16.5, 64^3 122 / 83.9 (580
 // MB of records: 6.9 TB/s of the 7.4 TB/s that a bare ring of copies reaches);
 // FP32 rows 64^3 96.6 / 61.8; 20-node bricks 4^3 - / 21.5 (27.9), 10^3 60 / 28.5, 21 x
-// 17 x 23 82 / 45.7, 32^3 205 / 136.  A phase of one tile per SM takes 1.4 us on a
+// 17 x 23 82 / 43.1, 32^3 205 / 136.  A phase of one tile per SM takes 1.4 us on a
 // small mesh: 0.3 us from the barrier to the published values, 0.9 us until the
 // neighbours hold them; of a cluster 1.1 us, of one tile 0.8 us, most of it the
 // dependent FP64 chain from the late columns to the point update.  Of the 64^3
@@ -637,7 +637,10 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
         // A phase's groups begin at the warp after the last one of the phase
         // before, so that the warps of a phase of few rows have taken their rows
         // while others finished the phase before (us per sweep with every phase
-        // beginning at warp 0: clusters 8^3 11.0, 20-node 4^3 27.9 against 9.0, 21.5).
+        // beginning at warp 0: clusters 8^3 11.0, 20-node 4^3 27.9 against 9.0, 21.5; 32^3
+        // 17.0 against 16.5).  Not in tiles that stream all their rows, whose phases
+        // have several groups a warp: 21 x 17 x 23 20-node bricks 43.1 against 45.7.
+        const bool rotate = CL || nring < nslots;
         int w0 = 0, g = s_seg[0] + warp * L::RPW, c1 = s_seg[1];
         for (int s = 1; s <= A.maxsw; ++s) {
             for (int c = 0; c < ncol; ++c) {
@@ -669,7 +672,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1) k_sor_flow(const FlowArgs<T> 
                     }
                 }
                 const int cn = last ? 0 : c + 1, sn = last ? s + 1 : s;
-                w0 = (w0 + (c1 - s_seg[c] + L::RPW - 1) / L::RPW) % CW;
+                if (rotate) w0 = (w0 + (c1 - s_seg[c] + L::RPW - 1) / L::RPW) % CW;
                 g = s_seg[cn] + (warp - w0 + (warp < w0 ? CW : 0)) * L::RPW;
                 c1 = s_seg[cn + 1];
                 if (L::AHEAD && A.early && !bad && g < c1 && sn <= A.maxsw) {
