@@ -192,6 +192,7 @@ struct fas_handle {
     cudaGraphExec_t sor32_graph = nullptr; // one refinement cycle of the FP32 form
     bool sor32_graph_sym = false;          // ... on the symmetric rows
     bool fp32_fresh = false;     // the last assembly ran in FAS_MODE_SOR_FP32
+    bool blk32_fresh = false;    // ... and wrote blk32 too
     // reductions and control
     std::vector<int> sor_boff, sor_nblk;       // FP64 colour grids and their partial offsets
     std::vector<int> sor_boff32, sor_nblk32;   // FP32 colour grids (smaller rings, more CTAs)
@@ -1614,6 +1615,17 @@ int launch_elem(fas_handle *h, int inc, int nit)
     return 0;
 }
 
+// The colour kernels' FP32 rows and the FP32 mirror of the correction.
+int ensure_colour32(fas_handle *h)
+{
+    if (!h->sor_d32.p) CKA(h->sor_d32.alloc(3 * (size_t)h->nnod));
+    if (!h->blk32.p) {
+        CKA(h->blk32.alloc((size_t)brow_of(h->slots) * h->nnod));
+        CK(h->blk32.zero(h->stream));
+    }
+    return 0;
+}
+
 // ELVALS (+ SUVALS when bc): element pass then row-gather assembly.
 // Returns the first element's FAFERR code in element order, if any.
 int ensure_fp32(fas_handle *h)
@@ -1624,13 +1636,9 @@ int ensure_fp32(fas_handle *h)
         CKA(h->sor_d.alloc(nd3));
         CKA(h->sor_r.alloc(nd3));
     }
-    if (!h->sor_d32.p && (!h->fl_ok32 || (h->mode & FAS_MODE_SOR_SYM))) CKA(h->sor_d32.alloc(nd3));
-    // the colour kernels' FP32 rows; the persistent kernel packs its own
-    if (!h->blk32.p && !h->fl_ok32) {
-        CKA(h->blk32.alloc((size_t)brow_of(h->slots) * h->nnod));
-        CK(h->blk32.zero(h->stream));
-    }
-    return 0;
+    if (!h->sor_d32.p && (h->mode & FAS_MODE_SOR_SYM)) CKA(h->sor_d32.alloc(nd3));
+    // the persistent kernel packs its own FP32 rows
+    return !h->fl_ok32 || (h->mode & FAS_MODE_SOR_COLOUR) ? ensure_colour32(h) : 0;
 }
 
 // Symmetric FP32 rows (FAS_MODE_SOR_SYM with FAS_MODE_SOR_FP32, 27-slot
@@ -1719,6 +1727,7 @@ int elvals_impl(fas_handle *h, int inc, int nit, bool bc)
         LAUNCHED(h);
         h->P.n_assembly++;
         h->fp32_fresh = (h->mode & FAS_MODE_SOR_FP32) && h->sor_d.p;
+        h->blk32_fresh = h->block().blk32 != nullptr;
         h->P.assembly_bytes += h->asm_bytes;
     }
     CK(cudaMemcpyAsync(h->hc->ekey, h->ekey.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -1927,7 +1936,7 @@ int ensure_fp32_graph(fas_handle *h, const BlockDev &B, double tolerl)
 // Whether the FP64 / FP32 solve runs as the persistent tile kernel.
 bool flow_on(const fas_handle *h, bool fp32)
 {
-    return h->fl_nt > 0 && (fp32 ? h->fl_ok32 && !h->sym_on : h->fl_ok64);
+    return h->fl_nt > 0 && !(h->mode & FAS_MODE_SOR_COLOUR) && (fp32 ? h->fl_ok32 && !h->sym_on : h->fl_ok64);
 }
 
 template <typename T> struct FlowBufs;
@@ -1970,7 +1979,7 @@ template <typename T> int ensure_flow(fas_handle *h)
 int prepare_solve(fas_handle *h)
 {
     if (int rc = ensure_fp32(h)) return rc;
-    if (h->fl_nt == 0) return 0;
+    if (h->fl_nt == 0 || (h->mode & FAS_MODE_SOR_COLOUR)) return 0;
     const bool fp32 = (h->mode & FAS_MODE_SOR_FP32) && !(h->sor_small && !(h->mode & FAS_MODE_SOR_GRID));
     if (fp32 && h->fl_ok32 && !(h->mode & FAS_MODE_SOR_SYM)) return ensure_flow<float>(h);
     return !fp32 && h->fl_ok64 ? ensure_flow<double>(h) : 0;
@@ -2079,36 +2088,27 @@ int facsls_flow(fas_handle *h, const BlockDev &B, double tolerl, bool fp32)
     return 0;
 }
 
-// FACSLS: rhs <- ddx, ddx <- 0, multicolour SOR sweeps until the relative
-// change drops below toler^2 or 1000 sweeps (Stif_sol.f90:173-213).
-int facsls_impl(fas_handle *h, int *sweeps, double *error)
+// FACSLS with one launch per colour: FP64 sweeps, or the FP32 form's cycles.
+// Leaves the verdict in h->hc->sor.
+int facsls_colour(fas_handle *h, const BlockDev &B, double tolerl, bool fp32)
 {
     cudaStream_t s = h->stream;
     const size_t nd3 = 3 * (size_t)h->nnod;
-    CK(cudaMemcpyAsync(h->rhs.p, h->ddx.p, nd3 * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemsetAsync(h->ddx.p, 0, nd3 * sizeof(double), s));
-    CK(cudaMemsetAsync(h->ekey.p + 1, 0xFF, sizeof(unsigned long long), s));
-    CK(cudaMemsetAsync(h->sorctl.p, 0, sizeof(SorCtl), s));
-    BlockDev B = h->block();
-    k_diag_check<<<nblocks(h->nnod, 256), 256, 0, s>>>(B, h->ekey.p + 1);
-    LAUNCHED(h);
-    CK(cudaMemcpyAsync(&h->hc->ekey[1], h->ekey.p + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (h->hc->ekey[1] != ~0ull) return 903;
-    const double tolerl = h->C.toler * h->C.toler;
-    const bool small = h->sor_small && !(h->mode & FAS_MODE_SOR_GRID);
-    const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->fp32_fresh;
-    h->sym_on = fp32 && h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM);
-    const bool flow = flow_on(h, fp32);
     int done = 0, chunk = 4;
-    if (flow) {
-        if (const int rc = facsls_flow(h, B, tolerl, fp32)) return rc;
-        done = 1000;
-    } else if (FAS_SOR_RCP) {
+    if (FAS_SOR_RCP) {
         k_rdiag<<<nblocks(h->nnod, 256), 256, 0, s>>>(B, h->rdiag.p);
         LAUNCHED(h);
     }
-    if (fp32 && !flow) {
+    if (fp32) {
+        if (!h->sym_on) {
+            if (int rc = ensure_colour32(h)) return rc;
+            if (!h->blk32_fresh) {   // the assembly left them to the persistent kernel's packing
+                const size_t n = (size_t)B.brow * B.R;
+                k_round_rows<<<nblocks((long long)n, 256), 256, 0, s>>>(n, h->blk.p, h->blk32.p);
+                LAUNCHED(h);
+                h->blk32_fresh = true;
+            }
+        }
         // x (= ddx) starts at 0, so the first residual is rhs itself
         CK(cudaMemcpyAsync(h->sor_r.p, h->rhs.p, nd3 * sizeof(double), cudaMemcpyDeviceToDevice, s));
         CK(cudaMemsetAsync(h->sor_d.p, 0, nd3 * sizeof(double), s));
@@ -2177,6 +2177,31 @@ int facsls_impl(fas_handle *h, int *sweeps, double *error)
         if (h->hc->sor.conv) break;
         chunk = std::min(chunk * 2, 64);
     }
+    return 0;
+}
+
+// FACSLS: rhs <- ddx, ddx <- 0, multicolour SOR sweeps until the relative
+// change drops below toler^2 or 1000 sweeps (Stif_sol.f90:173-213).
+int facsls_impl(fas_handle *h, int *sweeps, double *error)
+{
+    cudaStream_t s = h->stream;
+    const size_t nd3 = 3 * (size_t)h->nnod;
+    CK(cudaMemcpyAsync(h->rhs.p, h->ddx.p, nd3 * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemsetAsync(h->ddx.p, 0, nd3 * sizeof(double), s));
+    CK(cudaMemsetAsync(h->ekey.p + 1, 0xFF, sizeof(unsigned long long), s));
+    CK(cudaMemsetAsync(h->sorctl.p, 0, sizeof(SorCtl), s));
+    BlockDev B = h->block();
+    k_diag_check<<<nblocks(h->nnod, 256), 256, 0, s>>>(B, h->ekey.p + 1);
+    LAUNCHED(h);
+    CK(cudaMemcpyAsync(&h->hc->ekey[1], h->ekey.p + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    if (h->hc->ekey[1] != ~0ull) return 903;
+    const double tolerl = h->C.toler * h->C.toler;
+    const bool small = h->sor_small && !(h->mode & FAS_MODE_SOR_GRID);
+    const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->fp32_fresh;
+    h->sym_on = fp32 && h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM);
+    const bool flow = flow_on(h, fp32);
+    if (const int rc = flow ? facsls_flow(h, B, tolerl, fp32) : facsls_colour(h, B, tolerl, fp32)) return rc;
     settle_spans(h);
     const int nsw = h->hc->sor.sweeps;
     h->P.sor_sweeps += nsw;

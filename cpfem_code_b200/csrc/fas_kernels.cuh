@@ -1397,6 +1397,13 @@ __global__ void k_rdiag(BlockDev B, double *rdiag)
     for (int c = 0; c < 3; ++c) rdiag[3 * (size_t)p + c] = 1.0 / B.blk[B.bi(p, 0, 4 * c)];
 }
 
+// The colour kernels' FP32 rows from the assembled FP64 rows (the same layout).
+__global__ void k_round_rows(size_t n, const double *__restrict__ blk, float *__restrict__ blk32)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) blk32[i] = (float)blk[i];
+}
+
 // 903 test (Stif_sol.f90:183-185): first DOF whose diagonal entry is zero.
 __global__ void k_diag_check(BlockDev B, unsigned long long *firstbad)
 {
