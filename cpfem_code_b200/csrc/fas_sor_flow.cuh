@@ -58,7 +58,7 @@
 // dependent FP64 chain from the late columns to the point update.  Of the 64^3
 // phase's 10 us the copies take 9.4.
 //
-// Every wait is bounded.  A wait that gives up raises ctl->fault; a CTA
+// Every wait is bounded (FLOW_POLLS).  A wait that gives up raises ctl->fault; a CTA
 // leaves only at a barrier where all its warps agree, after its own copies
 // have landed.
 #pragma once
@@ -208,8 +208,13 @@ __device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, unsigned n)
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
 
-// Bound of the polls of one wait (a poll is at least an L2 round trip, and
-// sleeps after the first few): seconds, where a sweep takes microseconds.
+// Bound of the looks of one wait: seconds for a poll of another tile (an L2 round
+// trip and a sleep each), 0.1 s for a look at shared memory with a 20 ns sleep,
+// some tens of ms for one without, which waits for the CTA's own producer only;
+// a sweep takes 6 us to 0.2 ms.  None of them spans the time that another kernel
+// holds an SM: the CTAs of a cooperative launch, or of a cluster, start together
+// (a block of another stream that sat on one SM for 0.5, 6 and 15 s delayed the
+// whole solve by as much and changed no result).
 constexpr int FLOW_POLLS = 1 << 21;
 
 // Polls `p` until its tag is `tag`; false after the bound or once another

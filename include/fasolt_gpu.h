@@ -113,11 +113,11 @@ extern "C" {
                                      the mode changes                       */
 #define FAS_MODE_SOR_COLOUR 512u  /* solves with one launch per colour instead
                                      of the persistent launch, which needs a
-                                     whole SM for each of its tiles at the
-                                     same time: for a GPU on which other
-                                     streams hold SMs for seconds.  The FP64
-                                     solve's iterates agree to rounding, the
-                                     FP32 form's to the bit                 */
+                                     whole SM for each of its tiles and starts
+                                     once all of them are free: for a GPU on
+                                     which other streams hold SMs for long.
+                                     The FP64 solve's iterates agree to
+                                     rounding, the FP32 form's to the bit   */
 #define FAS_MODE_SOR_SYM    256u  /* with FAS_MODE_SOR_FP32 on 8-node meshes:
                                      the FP32 sweeps stream each off-diagonal
                                      block once (K_mn = K_nm^T), from the
