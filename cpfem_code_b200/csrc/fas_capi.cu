@@ -830,7 +830,7 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
         CK(dst.put(v.data(), v.size(), s));
         return 0;
     };
-    int rc = up(h->fl_trow, trow);
+    int rc = up(h->fl_trow, trow);   // no room even for these: the colour kernels
     if (!rc) rc = up(h->fl_seg, seg);
     if (!rc) rc = up(h->fl_hptr, hptr);
     if (!rc) rc = up(h->fl_hseg, hseg);
@@ -848,6 +848,10 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
     if (!rc && cluster) rc = up(h->fl_pptr, pptr);
     if (!rc && cluster) rc = up(h->fl_pdst, pdst);
     if (!rc && cluster) rc = up(h->fl_pfirst, pfirst);
+    if (rc == FAS_E_NOMEM) {
+        cudaGetLastError();
+        return 0;
+    }
     if (rc) return rc;
     CK(cudaStreamSynchronize(s));
     h->fl_nt = nt;
@@ -1941,12 +1945,14 @@ bool flow_on(const fas_handle *h, bool fp32)
 
 template <typename T> struct FlowBufs;
 template <> struct FlowBufs<double> {
+    static bool &ok(fas_handle *h) { return h->fl_ok64; }
     static DVec<unsigned char> &rec(fas_handle *h) { return h->fl_rec64; }
     static size_t bytes(fas_handle *h) { return h->fl_nrec64; }
     static unsigned *voff(fas_handle *h) { return h->fl_voff64.p; }
     static int *cptr(fas_handle *h) { return h->fl_cptr64.p; }
 };
 template <> struct FlowBufs<float> {
+    static bool &ok(fas_handle *h) { return h->fl_ok32; }
     static DVec<unsigned char> &rec(fas_handle *h) { return h->fl_rec32; }
     static size_t bytes(fas_handle *h) { return h->fl_nrec32; }
     static unsigned *voff(fas_handle *h) { return h->fl_voff32.p; }
@@ -1954,16 +1960,25 @@ template <> struct FlowBufs<float> {
 };
 
 // Buffers of the persistent solve in value type T, sized on its first use
-// and kept (the pattern is fixed), with the rows' index words.
+// and kept (the pattern is fixed), with the rows' index words.  Where the device
+// has no room for them (the records are as large as the assembled rows) the
+// handle's solves of this type take the colour kernels: flow_on tells.
 template <typename T> int ensure_flow(fas_handle *h)
 {
     using B = FlowBufs<T>;
     const size_t R = h->nnod;
-    if (!h->fl_old.p) CKA(h->fl_old.alloc(3 * R));
-    if (!h->fl_sync.p) CKA(h->fl_sync.alloc(3 * R + 8 * (size_t)h->fl_nt));
-    if (sizeof(T) == 4 && !h->fl_eoff.p) CKA(h->fl_eoff.alloc(R));
     if (B::rec(h).p) return 0;
-    CKA(B::rec(h).alloc(B::bytes(h)));
+    cudaError_t e = cudaSuccess;
+    if (!h->fl_old.p) e = h->fl_old.alloc(3 * R);
+    if (e == cudaSuccess && !h->fl_sync.p) e = h->fl_sync.alloc(3 * R + 8 * (size_t)h->fl_nt);
+    if (e == cudaSuccess && sizeof(T) == 4 && !h->fl_eoff.p) e = h->fl_eoff.alloc(R);
+    if (e == cudaSuccess) e = B::rec(h).alloc(B::bytes(h));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        B::ok(h) = false;
+        return 0;
+    }
+    CKA(e);
     return flow_shape(h->slots, [&](auto sl) -> int {
         k_flow_meta<T, sl()><<<nblocks((long long)R * FlowRow<T, sl()>::LPR, 256), 256, 0, h->stream>>>(
             (int)R, h->fl_lcol.p, h->fl_head.p, h->fl_from.p, B::voff(h), h->fl_tile.p, h->fl_trow.p, B::cptr(h),
@@ -1981,7 +1996,10 @@ int prepare_solve(fas_handle *h)
     if (int rc = ensure_fp32(h)) return rc;
     if (h->fl_nt == 0 || (h->mode & FAS_MODE_SOR_COLOUR)) return 0;
     const bool fp32 = (h->mode & FAS_MODE_SOR_FP32) && !(h->sor_small && !(h->mode & FAS_MODE_SOR_GRID));
-    if (fp32 && h->fl_ok32 && !(h->mode & FAS_MODE_SOR_SYM)) return ensure_flow<float>(h);
+    if (fp32 && h->fl_ok32 && !(h->mode & FAS_MODE_SOR_SYM)) {
+        if (int rc = ensure_flow<float>(h)) return rc;
+        return ensure_fp32(h);   // the colour kernels' buffers if there was no room
+    }
     return !fp32 && h->fl_ok64 ? ensure_flow<double>(h) : 0;
 }
 
@@ -2061,7 +2079,6 @@ int facsls_flow(fas_handle *h, const BlockDev &B, double tolerl, bool fp32)
 {
     cudaStream_t s = h->stream;
     if (!fp32) {
-        if (int rc = ensure_flow<double>(h)) return rc;
         if (int rc = flow_begin<double>(h, B)) return rc;
         Span sp(h, &h->P.ms_sor_colour);
         if (int rc = launch_flow<double>(h, h->ddx.p, 1000, tolerl)) return rc;
@@ -2071,7 +2088,6 @@ int facsls_flow(fas_handle *h, const BlockDev &B, double tolerl, bool fp32)
         CK(cudaStreamSynchronize(s));
         return 0;
     }
-    if (int rc = ensure_flow<float>(h)) return rc;
     if (int rc = flow_begin<float>(h, B)) return rc;
     int per_read = 1;
     for (int done = 0; done < 1000;) {
@@ -2200,8 +2216,9 @@ int facsls_impl(fas_handle *h, int *sweeps, double *error)
     const bool small = h->sor_small && !(h->mode & FAS_MODE_SOR_GRID);
     const bool fp32 = !small && (h->mode & FAS_MODE_SOR_FP32) && h->fp32_fresh;
     h->sym_on = fp32 && h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM);
-    const bool flow = flow_on(h, fp32);
-    if (const int rc = flow ? facsls_flow(h, B, tolerl, fp32) : facsls_colour(h, B, tolerl, fp32)) return rc;
+    if (flow_on(h, fp32))
+        if (int rc = fp32 ? ensure_flow<float>(h) : ensure_flow<double>(h)) return rc;
+    if (const int rc = flow_on(h, fp32) ? facsls_flow(h, B, tolerl, fp32) : facsls_colour(h, B, tolerl, fp32)) return rc;
     settle_spans(h);
     const int nsw = h->hc->sor.sweeps;
     h->P.sor_sweeps += nsw;
@@ -2466,8 +2483,10 @@ int ensure_inc_graph(fas_handle *h, int inc, cudaGraphExec_t *out)
     const bool fp32 = graph_fp32(h);
     h->sym_on = fp32 && h->sym_state == 1 && (h->mode & FAS_MODE_SOR_SYM);
     // the solve's and the work order's buffers are sized outside the capture
-    if (flow_on(h, fp32))
+    if (flow_on(h, fp32)) {
         if (int rc = fp32 ? ensure_flow<float>(h) : ensure_flow<double>(h)) return rc;
+        if (int rc = ensure_fp32(h)) return rc;   // the colour kernels' buffers if there was no room
+    }
     if (group_pass(h))
         if (int rc = ensure_group(h)) return rc;
     if (group_pass(h)) {
