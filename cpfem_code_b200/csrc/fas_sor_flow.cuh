@@ -91,7 +91,8 @@ constexpr int FLOW_CL_PBAR = FLOW_MAXCOL * 8, FLOW_CL_PART = FLOW_CL_PBAR + 32,
 // FP32: positions are the assembled rows' slots, on the lanes of the colour
 // kernels, so that the products are summed in their order: FP32 sums in
 // another order are as good, but not the same, and differ by 1e-7 in what
-// the refinement leaves.
+// the refinement leaves.  At least 4 and 8 lanes: take() reads a lane's index
+// words of a row held in registers 8 at most, and a row has 16 a lane at most.
 //
 // 27-slot rows store values by position with a fixed pitch, whose distance
 // in banks keeps the rows that a warp reads at once off each other's banks;
@@ -102,7 +103,8 @@ constexpr int FLOW_CL_PBAR = FLOW_MAXCOL * 8, FLOW_CL_PART = FLOW_CL_PBAR + 32,
 // 81-slot rows the next lane's the row's place in its chunk in 16-byte units.
 template <typename T, int S> struct FlowRow {
     static constexpr bool F32 = sizeof(T) == 4;
-    static constexpr int LPR = F32 ? tma_lpr<S, float>() : S == SLOTS ? 8 : 16;
+    static constexpr int LPR32 = tma_lpr<S, float>(), LEAST32 = S == SLOTS ? 4 : 8;
+    static constexpr int LPR = F32 ? (LPR32 > LEAST32 ? LPR32 : LEAST32) : S == SLOTS ? 8 : 16;
     static constexpr int SPL = (S + LPR - 1) / LPR;
     static constexpr int JL = F32 ? SPL : SPL - 2;       // first position round that may hold late columns
     static constexpr int LATE = F32 ? 0 : S - JL * LPR;
@@ -134,6 +136,7 @@ template <typename T, int S> struct FlowRow {
     static constexpr int SLOT = HB + CH * VB;
     static_assert(VB % 16 == 0 && MB % 16 == 0 && EB % 16 == 0, "bulk copies move 16-byte multiples");
     static_assert(HQ < LPR && (S == SLOTS || HQ + 1 < LPR) && SPL <= MW && LATE < 64, "header words");
+    static_assert(!AHEAD || MW <= 8, "take() reads 8 words at most");
     // where a column of position p is stored, for a row of ne early and nl late columns (-1: none)
     __host__ __device__ static constexpr int stored(int p, int ne, int nl)
     {
