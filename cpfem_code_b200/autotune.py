@@ -1,7 +1,10 @@
 """Autotuner of the kernels' launch shapes and scheduling options.
 
-Every knob is a set of compile-time defines, tuned on the workload whose
-time it sets:
+Every knob is a set of compile-time defines of the general kernels: the solve
+with one launch per colour and the constitutive pass with one thread per Gauss
+point, which serve what the persistent solve and the group pass do not take.
+Each is timed on those kernels (FAS_MODE_SOR_COLOUR; materials without a single
+latent hardening number):
 
 * ``sor27``: ``FAS_TMA_ROWS``, ``FAS_TMA_LPR``, ``FAS_TMA_STAGES`` (rows per
   chunk, lanes per row, ring stages of the 27-slot SOR colour kernel),
@@ -110,6 +113,15 @@ def _solve_us(p, reps: int = 3, mode: int = 0) -> tuple[float, int]:
         g.close()
 
 
+def _general(p):
+    """`p` with another latent hardening number for one pair of systems of every
+    material, which leaves it to the general constitutive kernels."""
+    p = p.copy()
+    p.smatrx = p.smatrx.copy()
+    p.smatrx[:, 0, 1] += 0.1
+    return p
+
+
 def _cp_ms(p, points: bool, reps: int = 5) -> float:
     """Constitutive-pass time: fas_gpu_constitutive on a point batch, or the
     element pass of ELVALS after one increment."""
@@ -138,21 +150,22 @@ def _cp_ms(p, points: bool, reps: int = 5) -> float:
 
 
 def measure() -> dict:
-    from . import generator
+    from . import abi, generator
     probs = dict(cube64=generator.workload("cube64"), brick20_32=generator.workload("brick20_32"),
-                 mixed32=generator.workload("mixed32"), points=generator.point_batch(1 << 20, seed=1))
+                 mixed32=_general(generator.workload("mixed32")), points=_general(generator.point_batch(1 << 20, seed=1)))
+    fp64, fp32 = abi.FAS_MODE_SOR_COLOUR, abi.FAS_MODE_SOR_COLOUR | abi.FAS_MODE_SOR_FP32
     out = {}
     for i in range(n_libs()):
         _load(lib_path(i))
         try:
-            us27, sw27 = _solve_us(probs["cube64"])
+            us27, sw27 = _solve_us(probs["cube64"], mode=fp64)
         except Exception as e:   # a combination the device refuses (e.g. a ring above its shared memory)
             out[str(i)] = dict(defines=defines_of(i), error=str(e))
             print(json.dumps(out[str(i)]), flush=True)
             continue
-        us81, sw81 = _solve_us(probs["brick20_32"])
-        us32, sw32 = _solve_us(probs["cube64"], mode=1)   # FAS_MODE_SOR_FP32
-        us8132, sw8132 = _solve_us(probs["brick20_32"], mode=1)
+        us81, sw81 = _solve_us(probs["brick20_32"], mode=fp64)
+        us32, sw32 = _solve_us(probs["cube64"], mode=fp32)
+        us8132, sw8132 = _solve_us(probs["brick20_32"], mode=fp32)
         out[str(i)] = dict(defines=defines_of(i), cube64_sweep_us=us27, cube64_sweeps=sw27,
                            brick20_32_sweep_us=us81, brick20_32_sweeps=sw81,
                            cube64_fp32_sweep_us=us32, cube64_fp32_sweeps=sw32,
