@@ -603,8 +603,9 @@ void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::v
 // nodes per CTA (one tile, a cluster of 16 or one per SM, by the rows' bytes), its rows by colour (rows that other tiles read first), the
 // tile-local index of every column, and the halo: the nodes of other tiles
 // that the tile's rows read, by colour.  A mesh with more colours than the
-// kernel's tables, or tiles whose solution values leave no room for a copy
-// ring (about 90^3 8-node bricks per GPU in FP64), keeps the colour kernels.
+// kernel's tables, or tiles whose solution values leave too little room for the
+// copy ring (FlowRow::LEAST: cubes beyond about 81^3 8-node or 45^3 20-node bricks,
+// in FP32 79^3 and 43^3), keeps the colour kernels.
 template <typename T, int S> bool flow_fits(int n, int nh, int ndst)
 {
     using L = FlowRow<T, S>;
@@ -612,7 +613,7 @@ template <typename T, int S> bool flow_fits(int n, int nh, int ndst)
     o += ndst >= 0 ? FLOW_CL_BYTES + (size_t)ndst * 4 + (size_t)(n + 1) * 2 : (size_t)nh * 4;
     o += (S == SLOTS ? 0 : (size_t)((n + L::CH - 1) / L::CH + 1) * 4);
     o = (o + 127) & ~(size_t)127;
-    return n + nh < 65536 && o + 3 * (size_t)L::SLOT <= (size_t)FLOW_SMEM;
+    return n + nh < 65536 && o + L::LEAST * (size_t)L::SLOT <= (size_t)FLOW_SMEM;
 }
 
 // f(slots) with the slots as a compile-time constant

@@ -134,6 +134,13 @@ template <typename T, int S> struct FlowRow {
     // chunk held the producer thread to 349 ns per chunk whatever its size)
     static constexpr int HB = CH * (MB + EB);
     static constexpr int SLOT = HB + CH * VB;
+    // Chunk slots that a tile's solution values must leave, or the colour kernels
+    // serve the mesh: the copies in flight no longer cover HBM's latency below (us
+    // per sweep of the colour kernels against this one with so many slots; 8-node
+    // cubes 80^3 233 / 208 (5), 82^3 242 / 262 (4), 86^3 282 / 411 (3); 20-node 44^3
+    // 457 / 416 (4), 46^3 525 / 605 (3); FP32 78^3 158 / 146 (4), 80^3 162 / 200 (3),
+    // 20-node 42^3 314 / 302 (4), 44^3 328 / 387 (3)).
+    static constexpr int LEAST = !F32 && S == SLOTS ? 5 : 4;
     static_assert(VB % 16 == 0 && MB % 16 == 0 && EB % 16 == 0, "bulk copies move 16-byte multiples");
     static_assert(HQ < LPR && (S == SLOTS || HQ + 1 < LPR) && SPL <= MW && LATE < 64, "header words");
     static_assert(!AHEAD || MW <= 8, "take() reads 8 words at most");
