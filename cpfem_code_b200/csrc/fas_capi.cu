@@ -412,16 +412,21 @@ int build_layout(fas_handle *h, const std::vector<double> &xyz)
     // shares an element with, ascending
     const int NN = h->nn;
     std::vector<std::vector<int>> nbs(nn);
+    std::vector<int> seen(nn, -1), at(nn, 0), others;   // the last row that met a node, and its slot there
     int maxs = 0;
     for (int p = 0; p < nn; ++p) {
         const int n = perm[p];
-        std::vector<int> others;
+        others.clear();
+        seen[n] = p;
         for (int k = h->ne_ptr[n]; k < h->ne_ptr[n + 1]; ++k) {
             const int e = h->ne_list[k];
             for (int a = 0; a < NN; ++a) {
                 const int m = h->h_ln[(size_t)e * NN + a];
                 if (m < 0) break;
-                if (m != n && std::find(others.begin(), others.end(), m) == others.end()) others.push_back(m);
+                if (seen[m] != p) {
+                    seen[m] = p;
+                    others.push_back(m);
+                }
             }
         }
         std::sort(others.begin(), others.end());
@@ -443,15 +448,16 @@ int build_layout(fas_handle *h, const std::vector<double> &xyz)
         bcol[(size_t)p * crow + h->slots] = cnt;   // the pad slot carries the slot count
         for (int s = 0; s < cnt; ++s) {
             bcol[(size_t)p * crow + s] = nbs[p][s];
-            unsigned long long *words = &bloc[((size_t)p * crow + s) * nbw];
-            int k = 0;
-            for (int q = h->ne_ptr[n]; q < h->ne_ptr[n + 1]; ++q, ++k) {
-                const int e = h->ne_list[q];
-                unsigned long long b = 0xFF;
-                for (int a = 0; a < NN; ++a)
-                    if (h->h_ln[(size_t)e * NN + a] == nbs[p][s]) { b = (unsigned long long)a; break; }
-                unsigned long long &word = words[k >> 3];
-                word = (word & ~(0xFFull << (8 * (k & 7)))) | (b << (8 * (k & 7)));
+            at[nbs[p][s]] = s;
+        }
+        // byte k of a slot's words: its node's first local index in the k-th adjacent element (0xFF: none)
+        int k = 0;
+        for (int q = h->ne_ptr[n]; q < h->ne_ptr[n + 1]; ++q, ++k) {
+            const int *ln = &h->h_ln[(size_t)h->ne_list[q] * NN];
+            const int sh = 8 * (k & 7);
+            for (int a = 0; a < NN && ln[a] >= 0; ++a) {
+                unsigned long long &word = bloc[((size_t)p * crow + at[ln[a]]) * nbw + (k >> 3)];
+                if ((word >> sh & 0xFF) == 0xFF) word = (word & ~(0xFFull << sh)) | ((unsigned long long)a << sh);
             }
         }
     }
@@ -538,7 +544,10 @@ int build_layout(fas_handle *h, const std::vector<double> &xyz)
     CK(h->d_cstart.put(h->col_start.data(), h->ncol + 1, s));
     h->sor_small = nn <= (h->slots == SLOTS ? SOR_SMALL_ROWS : SOR_SMALL_ROWS81);
     CK(cudaStreamSynchronize(s));
-    return build_flow(h, xyz, bcol, nslot, rowof);
+    const int rc = build_flow(h, xyz, bcol, nslot, rowof);
+    if (rc != FAS_E_NOMEM) return rc;
+    cudaGetLastError();              // no room for the tile layout: the colour kernels solve
+    return 0;
 }
 
 // Recursive coordinate bisection into nt tiles t0 .. t0 + nt - 1: cut across
@@ -831,7 +840,7 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
         CK(dst.put(v.data(), v.size(), s));
         return 0;
     };
-    int rc = up(h->fl_trow, trow);   // no room even for these: the colour kernels
+    int rc = up(h->fl_trow, trow);
     if (!rc) rc = up(h->fl_seg, seg);
     if (!rc) rc = up(h->fl_hptr, hptr);
     if (!rc) rc = up(h->fl_hseg, hseg);
@@ -849,10 +858,6 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
     if (!rc && cluster) rc = up(h->fl_pptr, pptr);
     if (!rc && cluster) rc = up(h->fl_pdst, pdst);
     if (!rc && cluster) rc = up(h->fl_pfirst, pfirst);
-    if (rc == FAS_E_NOMEM) {
-        cudaGetLastError();
-        return 0;
-    }
     if (rc) return rc;
     CK(cudaStreamSynchronize(s));
     h->fl_nt = nt;
