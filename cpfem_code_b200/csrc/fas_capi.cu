@@ -550,14 +550,40 @@ int build_layout(fas_handle *h, const std::vector<double> &xyz)
     return 0;
 }
 
+// Weights of the axes for the bisection: elements longer along one axis count
+// by their number there, not by their length, or a sheet of long elements would
+// be cut between its layers, with every node in its tile's halo (us per sweep of
+// 200 x 200 x 3 bricks of a unit cube 96.6, of 150 x 150 x 6 92.3; with the weights
+// 45.7 and 45.9; one launch per colour 80.8 and 78.0).  Elements within 1.5 of
+// the shortest count as equal.
+void axis_weights(const fas_handle *h, const std::vector<double> &xyz, double w[3])
+{
+    const int NN = h->nn, step = std::max(1, h->nlmnt / 4096);   // a sample tells
+    double len[3] = {0.0, 0.0, 0.0};
+    for (int e = 0; e < h->nlmnt; e += step) {
+        const int *ln = &h->h_ln[(size_t)e * NN];
+        if (ln[NN - 1] < 0) continue;   // a tie element
+        for (int d = 0; d < 3; ++d) {
+            double mn = 1e300, mx = -1e300;
+            for (int a = 0; a < NN; ++a) {
+                mn = std::min(mn, xyz[3 * (size_t)ln[a] + d]);
+                mx = std::max(mx, xyz[3 * (size_t)ln[a] + d]);
+            }
+            len[d] += mx - mn;
+        }
+    }
+    const double least = std::min(len[0], std::min(len[1], len[2]));
+    for (int d = 0; d < 3; ++d) w[d] = len[d] > 1.5 * least ? least / len[d] : 1.0;
+}
+
 // Recursive coordinate bisection into nt tiles t0 .. t0 + nt - 1: cut across
-// the longest extent of the bounding box, in proportion to the tiles on each
-// side.  Every colour's nodes (nodes[lo[c], hi[c])) are cut in that proportion
+// the longest (weighted) extent of the bounding box, in proportion to the tiles on
+// each side.  Every colour's nodes (nodes[lo[c], hi[c])) are cut in that proportion
 // by themselves, so that each tile has its share of every colour: a phase of
 // the solve handles one colour and is as long as its largest share.  `carry`
 // keeps the colours' rounding from adding up.
 void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::vector<int> &hi, int t0, int nt,
-               const std::vector<double> &xyz, bool by_colour, std::vector<int> &tile_of)
+               const std::vector<double> &xyz, const double w[3], bool by_colour, std::vector<int> &tile_of)
 {
     const int nc = (int)lo.size();
     if (nt <= 1) {
@@ -574,7 +600,7 @@ void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::v
             }
     int ax = 0;
     for (int d = 1; d < 3; ++d)
-        if (mx[d] - mn[d] > mx[ax] - mn[ax]) ax = d;
+        if (w[d] * (mx[d] - mn[d]) > w[ax] * (mx[ax] - mn[ax])) ax = d;
     const int ntl = nt / 2;
     std::vector<int> cut(nc);
     auto before = [&](int a, int b) {
@@ -604,8 +630,8 @@ void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::v
         if (cut[c] > lo[c] && cut[c] < hi[c])
             std::nth_element(nodes.begin() + lo[c], nodes.begin() + cut[c], nodes.begin() + hi[c], before);
     }
-    rcb_tiles(nodes, lo, cut, t0, ntl, xyz, by_colour, tile_of);
-    rcb_tiles(nodes, cut, hi, t0 + ntl, nt - ntl, xyz, by_colour, tile_of);
+    rcb_tiles(nodes, lo, cut, t0, ntl, xyz, w, by_colour, tile_of);
+    rcb_tiles(nodes, cut, hi, t0 + ntl, nt - ntl, xyz, w, by_colour, tile_of);
 }
 
 // Tile layout of the persistent SOR solve (k_sor_flow): one spatial tile of
@@ -706,7 +732,9 @@ int build_flow(fas_handle *h, const std::vector<double> &xyz, const std::vector<
     std::vector<int> nodes(nn), tile_of(nn, 0), clo(h->col_start.begin(), h->col_start.end() - 1),
         chi(h->col_start.begin() + 1, h->col_start.end());
     for (int m = 0; m < nn; ++m) nodes[rowof_host[m]] = m;   // by colour
-    rcb_tiles(nodes, clo, chi, 0, nt, xyz, nn < FLOW_EVEN_ROWS * nt, tile_of);
+    double w[3];
+    axis_weights(h, xyz, w);
+    rcb_tiles(nodes, clo, chi, 0, nt, xyz, w, nn < FLOW_EVEN_ROWS * nt, tile_of);
     std::vector<unsigned char> shared(nn, 0);   // the node is read by another tile
     for (int m = 0; m < nn; ++m) {
         const int *c = &bcol_host[(size_t)rowof_host[m] * crow];

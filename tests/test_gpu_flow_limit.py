@@ -14,7 +14,17 @@ FP32 = abi.FAS_MODE_SOR_FP32
                                                      (44, 20, 0, True), (46, 20, 0, False), (42, 20, FP32, True),
                                                      (44, 20, FP32, False)])
 def test_limit(n, nodes, mode, persistent):
-    p = generator.cube_config(n=n, ninc=1, grain=2, seed=1, nodes=nodes)
+    _check(generator.cube_config(n=n, ninc=1, grain=2, seed=1, nodes=nodes), mode, persistent)
+
+
+@pytest.mark.parametrize("n,nodes", [((400, 400, 1), 8), ((1, 300, 400), 8), ((160, 160, 1), 20), ((2, 20000, 2), 8)])
+def test_sheets_and_rods_of_long_elements(n, nodes):
+    """Tiles are cut by the number of elements along an axis, not by their length:
+    cut between the layers, these meshes' halos left no room for the ring."""
+    _check(generator.structured_cube(n=n, ninc=1, seed=1, nodes=nodes, xfree=1), 0, True)
+
+
+def _check(p, mode, persistent):
     p.ctrl.toler = 3e-3                        # some tens of sweeps
     out = []
     for m in (mode, mode | abi.FAS_MODE_SOR_COLOUR):
