@@ -826,6 +826,18 @@ def run_gpu_points(args, ws, rank, local, dist, dev):
     torch.cuda.synchronize()
     e2e = time.perf_counter() - t0
     te, work_e = reduce_max_sum(dist, e2e, float(prob.ngps * args.steps), dev)
+    # the plain kernel, one thread per point, which serves materials without a
+    # single latent hardening number: one pair of systems of the same points has another
+    other = start.copy()
+    other.smatrx = other.smatrx.copy()
+    other.smatrx[:, 0, 1] += 0.1
+    plain_ms = 0.0
+    with GpuSolver(other.copy()) as gp:
+        for k in range(args.warmup + args.steps):
+            gp.upload(other)
+            gp.profile(2)
+            gp.constitutive(1, 1)
+            plain_ms += gp.profile(0)["ms_constitutive"] if k >= args.warmup else 0.0
     if rank == 0:
         g.upload(start)
         g.constitutive(1, 1)
@@ -841,6 +853,10 @@ def run_gpu_points(args, ws, rank, local, dist, dev):
             "clocks": clk,
             "e2e": {"value": work_e / te, "unit": "GP-updates/s",
                     "h2d_bytes_per_step": moved_bytes(prob, 12), "d2h_bytes_per_step": moved_bytes(prob, 12)},
+            "persistent": {"ms_per_pass": ms / args.steps, "plain_ms_per_pass": plain_ms / args.steps,
+                           "mode": "groups of lanes on resident CTAs take points from a device queue (k_cp, the timed "
+                                   "pass); plain: one thread per point (k_points) on the same points with one pair of "
+                                   "systems' latent hardening raised by 0.1"},
         }
         if ws == 1 and not args.no_cpu:
             secs, pc = cpu_points(start, os.cpu_count() or 1)
