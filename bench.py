@@ -759,7 +759,7 @@ def run_gpu_diff16(args, ws, rank, local, dist, dev):
             "parallelism": f"replicas{ws}", "gpu_launches": int(prof["n_launches"]),
             "J": out["J"], "finite_difference_check": fd,
             "roofline": None,
-            "roofline_note": "the reverse kernel is bound by local-memory spills (profiles/k_replay_adj_points16k.md)",
+            "roofline_note": "k_cp and k_replay_rev are chains of dependent operations per point, a warp or two per scheduler",
             "clocks": clk,
             "e2e": {"value": work_e / te, "unit": "GP-increments/s",
                     "h2d_bytes_per_step": int(hist.de.nbytes + hist.dr.nbytes + hist.w.nbytes + hist.y.nbytes),

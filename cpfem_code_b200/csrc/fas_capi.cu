@@ -274,7 +274,8 @@ struct fas_handle {
     }
 };
 
-// meshes with at most this many nodes run each SOR solve in one CTA: 256
+// meshes with at most this many nodes run fas_gpu_facsls_noalloc in one CTA
+// (k_sor_small) and solve in FP64 unless FAS_MODE_SOR_GRID is set: 256
 // for 27-slot rows (1024 threads, a slot per lane; measured us per sweep,
 // one CTA against the colour kernels: 17 / 33 at 125 nodes, 74 / 27 at
 // 729, 439 / 26 at 4,913); 512 for 81-slot rows, whose three slots per lane
@@ -635,8 +636,8 @@ void rcb_tiles(std::vector<int> &nodes, const std::vector<int> &lo, const std::v
 }
 
 // Tile layout of the persistent SOR solve (k_sor_flow): one spatial tile of
-// nodes per CTA (one tile, a cluster of 16 or one per SM, by the rows' bytes), its rows by colour (rows that other tiles read first), the
-// tile-local index of every column, and the halo: the nodes of other tiles
+// nodes per CTA (one tile, a cluster of 16 or one per SM, by the rows' bytes),
+// its rows by colour (rows that other tiles read first), the tile-local index of every column, and the halo: the nodes of other tiles
 // that the tile's rows read, by colour.  A mesh with more colours than the
 // kernel's tables, or tiles whose solution values leave too little room for the
 // copy ring (FlowRow::LEAST: cubes beyond about 81^3 8-node or 45^3 20-node bricks,
@@ -1217,7 +1218,7 @@ int create_impl(fas_handle *h, const fas_mesh_desc *Md, const fas_matl_desc *T, 
     // the group pass serves materials with one latent hardening number q and
     // self hardening not below it, positive rate exponents and hardening
     // coefficients not below zero: what its formula needs (fas_cp_group.cuh).
-    // It is faster at every size (27 points 0.07 against 0.61 ms, 2^20 points 11.6
+    // It is faster at every size (27 points 0.07 against 0.61 ms, 2^20 points 12.4
     // against 28.2 ms), so that size does not enter the rule
     std::vector<char> one(nm, 1);
     for (int m = 0; m < nm; ++m) {
@@ -2771,7 +2772,7 @@ void launch_replay_adj(fas_handle *h, const ReplayDev &H, const DevGp &G, int rs
 
 // The replay by groups of lanes (fas_replay_group.cuh): its buffers, or
 // `ready` false where the materials or the memory left call for a thread per GP.
-// The rule is the group pass's: 4,096 points and 20 increments 9.6 against 147 ms,
+// The rule is the group pass's: 4,096 points and 20 increments 9.9 against 147 ms,
 // one increment of as
 // many points 0.75 against 3.6.
 int replay_group_prepare(fas_handle *h, const fas_replay_desc *d, DevGp &G, bool &ready)

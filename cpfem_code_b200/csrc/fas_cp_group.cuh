@@ -6,7 +6,9 @@
 // run-time indices: a point's chain of dependent loads took 1.7 ms however few
 // points there were, and 2^20 points 28 ms (0.6 TFLOP/s of FP64).  Here
 //   * L lanes serve a point, lane l the slip systems l, l + L, ...: 3 or 4 per
-//     lane, so that everything stays in registers with compile-time indices;
+//     lane, with compile-time indices instead of scratch behind run-time ones.  At
+//     the 128 registers that four CTAs an SM leave, 1.3 KB (12 systems) to 1.7 KB
+//     (32) a thread are still spilled, most of it around the 6 x 6 matrix;
 //   * smatrx(i, j) = q for i /= j and its diagonal d_i >= q make the two
 //     matrices of the local problem diagonal plus rank one, and the elimination
 //     without pivoting of FACTOR and SOLVER (src/fasolt/crys-cons.f90:244-309)
@@ -27,7 +29,7 @@
 // in lockstep, an outer iteration of each at a time.
 //
 // Constitutive pass before and after: 4,096 FCC points 1.75 and 0.20 ms,
-// 100,003 HCP points 5.8 and 3.1 ms, 2^20 FCC points 28.2 and 12.2 ms, a 64^3
+// 100,003 HCP points 5.8 and 3.1 ms, 2^20 FCC points 28.2 and 12.4 ms, a 64^3
 // mesh 11 and 2.7 ms.  The iterations are bound by their dependent chains of
 // sums, logarithms and divisions (0.3 instructions a cycle and scheduler at 15
 // warps an SM), and by fetching their code.  Against the same update in more

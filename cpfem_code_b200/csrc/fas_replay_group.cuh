@@ -16,9 +16,11 @@
 //   * the derivatives by the Euler angles go through the direction cosines a:
 //     abar collects what the slip systems, ELASTC and ECHROT pass back.
 // The matrices are those of the dual passes, in another order of summation.
-// 4,096 points and 20 increments now take 9.6 ms with segments of five: 35
+// 4,096 points and 20 increments now take 9.9 ms with segments of five: 35
 // increments forwards at 0.25 ms (k_cp 0.23), four segments backwards at 0.11 ms.
-// Both are one dependent chain per point with a warp or two per scheduler.  The
+// Both are one dependent chain per point with a warp or two per scheduler, at 128
+// and 255 registers with spills (k_replay_rev: 1.8 KB stored for 12 systems, 3.1 for
+// 32).  The
 // gradient's error against the same in more digits went from 8.9e-13 to 5.8e-13.
 #pragma once
 
